@@ -47,11 +47,7 @@ NCU_FP64_PIPE_ACTIVE = {1024: 0.435}
 
 def step_kernel_name(variant):
     """The unsplit step kernel a launch variant runs (claw2_tune_set)."""
-    if variant == 8:
-        return "k_step_unsplit_ws<RPEulerRoe,128>"
-    if variant == 4:
-        return "k_step_unsplit2<RPEulerRoe,128>"
-    return "k_step_unsplit%s<RPEulerRoe,128,%d>" % ("_tma" if variant & 2 else "", 3 if variant & 1 else 2)
+    return "k_step_unsplit%s<RPEulerRoe,128,%d>" % ("_tma" if variant in (2, 3) else "", 3 if variant in (1, 3) else 2)
 
 
 def parse():

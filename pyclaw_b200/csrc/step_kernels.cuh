@@ -84,17 +84,51 @@ __device__ __forceinline__ int tile_index(const StepArgs& a) {
     return tile;
 }
 
-// philim.f90:16-35
-__device__ __forceinline__ double philim(double a, double b, int meth) {
-    const double r = b * rcp_nr(a);
-    switch (meth) {
-        case 1: return fmax(0.0, fmin(1.0, r));
-        case 2: return fmax(0.0, fmax(fmin(1.0, 2.0 * r), fmin(2.0, r)));
-        case 3: return (r + fabs(r)) / (1.0 + fabs(r));
-        case 4: return fmax(0.0, fmin((1.0 + r) / 2.0, fmin(2.0, 2.0 * r)));
-        case 5: return r;
-        default: return 0.0;
+// The limiter function of philim.f90:16-35 at the ratio r = num / den.
+//
+// No test for a zero wave (limiter.f90:42 skips those): phi multiplies that
+// wave, so any finite value will do, and every branch below is bounded
+// whatever the ratio (a zero or subnormal den gives a reciprocal of +-inf and a
+// NaN ratio).  Comparisons that the ratio's sign bit or exponent decides are
+// integer instructions, off the FP64 pipe that bounds the kernels.  Van Leer's
+// (r + |r|) / (1 + |r|) is 2 |num| / (|num| + |den|) for r > 0: the form with
+// the ratio is inf / inf where the neighbour's wave outgrows this one by more
+// than the range of a double.
+__device__ __forceinline__ double philim(double num, double den, int meth) {
+    if (meth == 3) {
+        const double an = fabs(num), x = an * rcp_nr(an + fabs(den));
+        const double phi = x + x;
+        return (__double2hiint(num) ^ __double2hiint(den)) < 0 ? 0.0 : (phi < 2.0 ? phi : 2.0);
     }
+    if (meth == 5) {
+        const double r = num * rcp_nr(den);
+        return fabs(r) < 1e300 ? r : 1.0;
+    }
+    double r0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(den));
+    double e = fma(-den, r0, 1.0);
+    double ri = fma(r0, e, r0);
+    e = fma(-den, ri, 1.0);
+    ri = fma(ri, e, ri);  // rcp_nr without its special values
+    const double r = num * ri;
+    const bool neg = __double2hiint(r) < 0;
+    double phi;
+    switch (meth) {
+        case 1: phi = r < 1.0 ? r : 1.0; break;
+        case 2: {
+            const double lo = (r + r) < 1.0 ? r + r : 1.0, hi = r < 2.0 ? r : 2.0;
+            phi = lo > hi ? lo : hi;
+            break;
+        }
+        case 4: {
+            const double mean = 0.5 + 0.5 * r, twice = r + r;
+            phi = twice < mean ? twice : mean;
+            phi = __double2hiint(phi) < 0x40000000 ? phi : 2.0;  // (phi < 2 for phi >= 0; a NaN gives 2)
+            break;
+        }
+        default: phi = 0.0; break;
+    }
+    return neg ? 0.0 : phi;
 }
 
 __device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned long long* slot) {
@@ -151,44 +185,33 @@ __device__ __forceinline__ bool all_finite(const double (&v)[ME]) {
 enum { SPEC_ANY = 0, SPEC_MC2 = 1, SPEC_MM2 = 2 };
 
 // Limiter (limiter.f90:29-53 / philim.f90) and second-order correction
-// cqxx = sum_k coef_k * phi_k * w_k (flux2.f90:134-160) for one interface.
-// dl / dr are the dot products of each unlimited wave with the same family's
-// unlimited wave at the interface below/left and above/right.
+// cqxx = sum_k coef_k * phi_k * w_k (flux2.f90:134-160) for one interface with
+// limiter record `rec` (Lim<RP>).  num: per family, amplitude of the upwind
+// neighbour's wave times its dot product with this interface's eigenvector.
 template <class RP, int IXY, int SPEC = SPEC_ANY>
 __device__ __forceinline__ void correction(const typename RP::Iface& f, const RPParams& p, const Method& meth,
-                                           double dtdx, const double (&dl)[RP::MWAVES],
-                                           const double (&dr)[RP::MWAVES], double (&cq)[RP::MEQN]) {
-    constexpr int ME = RP::MEQN, MW = RP::MWAVES;
-    double s[MW];
-    RP::template speeds<IXY>(f, p, s);
-    double w[MW][ME];
-    RP::template waves<IXY>(f, p, w);
-#pragma unroll
-    for (int m = 0; m < ME; ++m) cq[m] = 0.0;
+                                           double dtdx, const double (&rec)[Lim<RP>::N],
+                                           const double (&s)[RP::MWAVES], const double (&num)[RP::MWAVES],
+                                           double (&cq)[RP::MEQN]) {
+    constexpr int MW = RP::MWAVES;
+    double X[MW], b[MW];
+    Lim<RP>::cross(rec, rec, X);
 #pragma unroll
     for (int k = 0; k < MW; ++k) {
         const int lim = (SPEC == SPEC_MC2) ? 4 : (SPEC == SPEC_MM2) ? 1 : meth.mthlim[k];
-        double wn2 = 0.0;
-#pragma unroll
-        for (int m = 0; m < ME; ++m) wn2 = wn2 + w[k][m] * w[k][m];
-        double phi = 1.0;
-        if (lim != 0 && wn2 != 0.0) phi = philim(wn2, (s[k] > 0.0) ? dl[k] : dr[k], lim);
+        const double amp = Lim<RP>::amp(rec, k);
+        const double phi = lim != 0 ? philim(num[k], amp * X[k], lim) : 1.0;
         const double as = fabs(s[k]);
         const bool fw = (SPEC != SPEC_ANY) ? false : (meth.fwave != 0);
         const double coef = (fw ? copysign(1.0, s[k]) : as) * (1.0 - as * dtdx);
-#pragma unroll
-        for (int m = 0; m < ME; ++m) cq[m] = cq[m] + coef * (phi * w[k][m]);
+        b[k] = coef * (phi * amp);
     }
+    Lim<RP>::template sum<IXY>(f, p, rec, b, cq);
 }
 
 template <class RP, int IXY>
 __device__ __forceinline__ double iface_cfl(const typename RP::Iface& f, const RPParams& p, double dtdx) {
-    double s[RP::MWAVES];
-    RP::template speeds<IXY>(f, p, s);
-    double c = 0.0;
-#pragma unroll
-    for (int k = 0; k < RP::MWAVES; ++k) c = fmax(c, fabs(dtdx * s[k]));
-    return c;
+    return dtdx * MaxSpeed<RP>::template get<IXY>(f, p);
 }
 
 // With a capacity function the two sides of an interface have their own
@@ -256,6 +279,20 @@ __device__ __forceinline__ void tma_row(const CUtensorMap* tm, double* dst, unsi
         : "memory");
 }
 
+// h times the transverse split of a solver whose rpt2 reads the cells beside
+// the receiving one.
+template <class RP, int IXY>
+__device__ __forceinline__ void rpt2h_aux(const double (&asdq)[RP::MEQN], const double (&cm)[RP::NC],
+                                          const double (&c0)[RP::NC], const double (&cp)[RP::NC], double h,
+                                          double (&bm)[RP::MEQN], double (&bp)[RP::MEQN]) {
+    RP::template rpt2_aux<IXY>(asdq, cm, c0, cp, bm, bp);
+#pragma unroll
+    for (int m = 0; m < RP::MEQN; ++m) {
+        bm[m] = h * bm[m];
+        bp[m] = h * bp[m];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Unsplit step (step2.f90), fused x + y sweeps.
 // ---------------------------------------------------------------------------
@@ -268,7 +305,7 @@ struct UnsplitSmem {
     static constexpr int NF = (int)(sizeof(typename RP::Iface) / sizeof(double));
     static constexpr bool YS = NF > 12;
     double cell[3][NC][NT];  // prepared cells of rows R-2, R-1, R (ring)
-    double w[MW][ME][NT];    // unlimited x-waves of row R
+    double w[Lim<RP>::N][NT];  // limiter records of row R's x-interfaces
     double xl[4][ME][NT];    // increments for column cp-1: rows R-2, R-1, R, R+1
     double yr[2][ME][NT];    // increments for column cp+1: rows R-2, R-1
     double icap[CAPA ? 3 : 1][CAPA ? NT : 1];  // 1 / kappa of the ring's cells (capacity form)
@@ -444,12 +481,12 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                     c0[k] = S.cell[s1][k][tl];
                     cu[k] = S.cell[s2][k][tl];
                 }
-                RP::template rpt2_aux<1>(cxa1, cm, c0, cu, bm, bp);  // imp = 1 -> column cp-1
+                rpt2h_aux<RP, 1>(cxa1, cm, c0, cu, hl, bm, bp);  // imp = 1 -> column cp-1
 #pragma unroll
                 for (int m = 0; m < ME; ++m) {
-                    dxl1[m] = hl * (bp[m] - bm[m]);
-                    dxl0[m] = hl * bm[m];
-                    dxl2[m] = -hl * bp[m];
+                    dxl1[m] = bp[m] - bm[m];
+                    dxl0[m] = bm[m];
+                    dxl2[m] = -bp[m];
                 }
 #pragma unroll
                 for (int k = 0; k < NC; ++k) {
@@ -457,12 +494,12 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                     c0[k] = S.cell[s1][k][t];
                     cu[k] = S.cell[s2][k][t];
                 }
-                RP::template rpt2_aux<1>(cxa2, cm, c0, cu, bm, bp);  // imp = 2 -> column cp
+                rpt2h_aux<RP, 1>(cxa2, cm, c0, cu, hr, bm, bp);  // imp = 2 -> column cp
 #pragma unroll
                 for (int m = 0; m < ME; ++m) {
-                    accB[m] = accB[m] + hr * (bp[m] - bm[m]);
-                    accA[m] = accA[m] + hr * bm[m];
-                    accC[m] = accC[m] - hr * bp[m];
+                    accB[m] = accB[m] + (bp[m] - bm[m]);
+                    accA[m] = accA[m] + bm[m];
+                    accC[m] = accC[m] - bp[m];
                 }
             }
             cx_valid = false;
@@ -494,14 +531,15 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
             }
             Iface fN;
             double amN[ME], apN[ME];
-            double dn[MW];
+            double dn[MW];  // limiter numerators of (R-1 | R) from (R-2 | R-1), and da the other way round
+            double da[MW];
             const bool zN = zs && __all_sync(0xffffffffu, same_q<ME, NC>(cB, cA));
             if (ZS && zN) {
                 SkipTraits<RP>::template zero_iface<2>(cB, cA, P, fN);
 #pragma unroll
                 for (int m = 0; m < ME; ++m) amN[m] = apN[m] = 0.0;
 #pragma unroll
-                for (int k = 0; k < MW; ++k) dn[k] = 0.0;
+                for (int k = 0; k < MW; ++k) dn[k] = da[k] = 0.0;
                 if (GuessTraits<RP>::USES && cp <= mx + 3) n_solve += 1;  // a solve with no Newton step
             } else {
                 double gy = 0.0;
@@ -512,15 +550,14 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                     n_app += GuessTraits<RP>::count_applied(fN);
                     n_solve += 1;
                 }
-                double wY[MW][ME], wN[MW][ME];
-                RP::template waves<2>(fY, P, wY);
-                RP::template waves<2>(fN, P, wN);
+                double rY[Lim<RP>::N], rN[Lim<RP>::N], X[MW];
+                Lim<RP>::template rec<2>(fY, P, rY);
+                Lim<RP>::template rec<2>(fN, P, rN);
+                Lim<RP>::cross(rY, rN, X);
 #pragma unroll
                 for (int k = 0; k < MW; ++k) {
-                    double d = 0.0;
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) d = d + wY[k][m] * wN[k][m];
-                    dn[k] = d;
+                    dn[k] = Lim<RP>::amp(rY, k) * X[k];
+                    da[k] = Lim<RP>::amp(rN, k) * X[k];
                 }
             }
             if (R >= R0 + 3) {
@@ -533,7 +570,12 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                 const double ydl = CAPA ? dtdy * S.icap[s0][t] : dtdy, ydr = CAPA ? dtdy * S.icap[s1][t] : dtdy;
                 double cq[ME];
                 if (order != 1) {
-                    correction<RP, 2, SPEC>(fY, P, a.meth, CAPA ? 0.5 * (ydl + ydr) : dtdy, dY, dn, cq);
+                    double rY[Lim<RP>::N], sY[MW], num[MW];
+                    Lim<RP>::template rec<2>(fY, P, rY);
+                    RP::template speeds<2>(fY, P, sY);
+#pragma unroll
+                    for (int k = 0; k < MW; ++k) num[k] = (sY[k] > 0.0) ? dY[k] : da[k];
+                    correction<RP, 2, SPEC>(fY, P, a.meth, CAPA ? 0.5 * (ydl + ydr) : dtdy, rY, sY, num, cq);
                 } else {
 #pragma unroll
                     for (int m = 0; m < ME; ++m) cq[m] = 0.0;
@@ -558,15 +600,15 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                             c0[k] = S.cell[s0][k][t];
                             cu[k] = S.cell[s0][k][tr];
                         }
-                        RP::template rpt2_aux<2>(as2, cm, c0, cu, bm, bp);
+                        rpt2h_aux<RP, 2>(as2, cm, c0, cu, hl, bm, bp);
                     } else {
-                        RP::template rpt2<2>(fY, P, as2, bm, bp);  // imp = 1 -> row R-2
+                        Trans<RP>::template split<2>(fY, P, hl, as2, bm, bp);  // imp = 1 -> row R-2
                     }
 #pragma unroll
                     for (int m = 0; m < ME; ++m) {
-                        accA[m] = accA[m] + hl * (bp[m] - bm[m]);
-                        ylB[m] = hl * bm[m];
-                        yrB[m] = -hl * bp[m];
+                        accA[m] = accA[m] + (bp[m] - bm[m]);
+                        ylB[m] = bm[m];
+                        yrB[m] = -bp[m];
                     }
 #pragma unroll
                     for (int m = 0; m < ME; ++m) as2[m] = tc ? apY[m] - cq[m] : apY[m];
@@ -578,15 +620,15 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                             c0[k] = S.cell[s1][k][t];
                             cu[k] = S.cell[s1][k][tr];
                         }
-                        RP::template rpt2_aux<2>(as2, cm, c0, cu, bm, bp);
+                        rpt2h_aux<RP, 2>(as2, cm, c0, cu, hr, bm, bp);
                     } else {
-                        RP::template rpt2<2>(fY, P, as2, bm, bp);  // imp = 2 -> row R-1
+                        Trans<RP>::template split<2>(fY, P, hr, as2, bm, bp);  // imp = 2 -> row R-1
                     }
 #pragma unroll
                     for (int m = 0; m < ME; ++m) {
-                        accB[m] = accB[m] + hr * (bp[m] - bm[m]);
-                        ylA[m] = hr * bm[m];
-                        yrA[m] = -hr * bp[m];
+                        accB[m] = accB[m] + (bp[m] - bm[m]);
+                        ylA[m] = bm[m];
+                        yrA[m] = -bp[m];
                     }
                 }
             }
@@ -639,28 +681,22 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                 if (GuessTraits<RP>::USES && xrow && cp <= mx + 3 && t > 0) n_solve += 1;
 #pragma unroll
                 for (int m = 0; m < ME; ++m) amX[m] = apX[m] = 0.0;
-#pragma unroll
-                for (int k = 0; k < MW; ++k)
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) S.w[k][m][t] = 0.0;
             } else {
-            double gx = 0.0;
-            if (GuessTraits<RP>::USES && a.guess) gx = a.guess[(long long)R * pitch + cpl];
-            GuessTraits<RP>::template solve<1>(cL, cR, P, gx, fX, amX, apX);
-            if (GuessTraits<RP>::USES && cp <= mx + 3 && t > 0) {
-                n_it += GuessTraits<RP>::count(fX);
-                n_app += GuessTraits<RP>::count_applied(fX);
-                n_solve += 1;
+                double gx = 0.0;
+                if (GuessTraits<RP>::USES && a.guess) gx = a.guess[(long long)R * pitch + cpl];
+                GuessTraits<RP>::template solve<1>(cL, cR, P, gx, fX, amX, apX);
+                if (GuessTraits<RP>::USES && cp <= mx + 3 && t > 0) {
+                    n_it += GuessTraits<RP>::count(fX);
+                    n_app += GuessTraits<RP>::count_applied(fX);
+                    n_solve += 1;
+                }
             }
-            double wX[MW][ME];
-            RP::template waves<1>(fX, P, wX);
+            double rX[Lim<RP>::N];
+            Lim<RP>::template rec<1>(fX, P, rX);
 #pragma unroll
-            for (int k = 0; k < MW; ++k)
-#pragma unroll
-                for (int m = 0; m < ME; ++m) S.w[k][m][t] = wX[k][m];
-            }
+            for (int k = 0; k < Lim<RP>::N; ++k) S.w[k][t] = rX[k];
         }
-        __syncthreads();  // S2: x-waves of row R visible
+        __syncthreads();  // S2: limiter records of row R visible
 
         double xcL[ME], xbL[ME], xaL[ME];
 #pragma unroll
@@ -674,20 +710,11 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
             const double xdl = CAPA ? dtdx * S.icap[s2][tl] : dtdx, xdr = CAPA ? dtdx * S.icap[s2][t] : dtdx;
             double cq[ME];
             if (order != 1) {
-                double dl[MW], dr[MW];
-#pragma unroll
-                for (int k = 0; k < MW; ++k) {
-                    double x = 0.0, y = 0.0;
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) {
-                        const double w = S.w[k][m][t];
-                        x = x + S.w[k][m][tl] * w;
-                        y = y + w * S.w[k][m][tr];
-                    }
-                    dl[k] = x;
-                    dr[k] = y;
-                }
-                correction<RP, 1, SPEC>(fX, P, a.meth, CAPA ? 0.5 * (xdl + xdr) : dtdx, dl, dr, cq);
+                double rX[Lim<RP>::N], sX[MW], num[MW];
+                Lim<RP>::template rec<1>(fX, P, rX);
+                RP::template speeds<1>(fX, P, sX);
+                Lim<RP>::up(rX, sX, [&](int j, bool left) { return S.w[j][left ? tl : tr]; }, num);
+                correction<RP, 1, SPEC>(fX, P, a.meth, CAPA ? 0.5 * (xdl + xdr) : dtdx, rX, sX, num, cq);
             } else {
 #pragma unroll
                 for (int m = 0; m < ME; ++m) cq[m] = 0.0;
@@ -713,21 +740,21 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                 double as2[ME], bm[ME], bp[ME];
 #pragma unroll
                 for (int m = 0; m < ME; ++m) as2[m] = tc ? amX[m] + cq[m] : amX[m];
-                RP::template rpt2<1>(fX, P, as2, bm, bp);  // imp = 1 -> column cp-1
+                Trans<RP>::template split<1>(fX, P, hl, as2, bm, bp);  // imp = 1 -> column cp-1
 #pragma unroll
                 for (int m = 0; m < ME; ++m) {
-                    xcL[m] = xcL[m] + hl * (bp[m] - bm[m]);
-                    xbL[m] = hl * bm[m];
-                    xaL[m] = -hl * bp[m];
+                    xcL[m] = xcL[m] + (bp[m] - bm[m]);
+                    xbL[m] = bm[m];
+                    xaL[m] = -bp[m];
                 }
 #pragma unroll
                 for (int m = 0; m < ME; ++m) as2[m] = tc ? apX[m] - cq[m] : apX[m];
-                RP::template rpt2<1>(fX, P, as2, bm, bp);  // imp = 2 -> column cp
+                Trans<RP>::template split<1>(fX, P, hr, as2, bm, bp);  // imp = 2 -> column cp
 #pragma unroll
                 for (int m = 0; m < ME; ++m) {
-                    accC[m] = accC[m] + hr * (bp[m] - bm[m]);
-                    accB[m] = accB[m] + hr * bm[m];
-                    accD[m] = accD[m] - hr * bp[m];
+                    accC[m] = accC[m] + (bp[m] - bm[m]);
+                    accB[m] = accB[m] + bm[m];
+                    accD[m] = accD[m] - bp[m];
                 }
             }
         }
@@ -769,812 +796,6 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
         s2 = tmp;
     }
     if (GuessTraits<RP>::USES && a.counters) counter_commit(a.counters, n_it, n_solve, n_app);
-}
-
-// ---------------------------------------------------------------------------
-// The two-barrier form of the tile ("deferred x finish").  Each x-interface
-// is solved on its row R as before, but finished (limiter with the
-// neighbours' waves, correction, transverse solves) one row later, together
-// with the y work of that row: at row R every thread
-//   * finishes the x-interface (cp-1 | cp) of row R-1 (its waves and those of
-//     the neighbours wait in a double-buffered shared array, its own record
-//     in shared memory), with the cells of rows R-2, R-1, R in the ring, so
-//     solvers whose transverse solve reads the neighbouring cells need no
-//     extra deferral,
-//   * solves the y-interface (R-1 | R) and finishes (R-2 | R-1),
-//   * solves the x-interface of row R and stores its waves,
-// all between the same two barriers (cells visible; increments visible).  The
-// three independent chains in one block give the scheduler independent
-// FP64 work, and a barrier per row is saved.  Every increment lands in the
-// same cell with the same factors as in unsplit_tile; row R-2 is still
-// complete and written at the end of row R.
-// ---------------------------------------------------------------------------
-template <class RP, int NT, bool CAPA = false>
-struct UnsplitSmem2 {
-    static constexpr int ME = RP::MEQN, MW = RP::MWAVES, NC = RP::NC;
-    static constexpr int NF = (int)(sizeof(typename RP::Iface) / sizeof(double)) + 2 * ME;  // record + A-dq, A+dq
-    double cell[3][NC][NT];   // prepared cells of rows R-2, R-1, R (ring)
-    double w[2][MW][ME][NT];  // unlimited x-waves of rows R-1 and R (by row parity)
-    double fx[NF][NT];        // this column's x-interface of row R-1: record, A-dq, A+dq
-    double xl[3][ME][NT];     // increments for column cp-1: rows R-2, R-1, R
-    double yr[2][ME][NT];     // increments for column cp+1: rows R-2, R-1
-    double icap[CAPA ? 3 : 1][CAPA ? NT : 1];
-    double red[NT / 32];
-};
-
-template <class RP, int NT, int SPEC = SPEC_ANY, bool CAPA = false, bool EVO = false>
-__device__ __forceinline__ void unsplit_tile2(const StepArgs& a, int strip, int rb, UnsplitSmem2<RP, NT, CAPA>& S,
-                                              double& cfl) {
-    constexpr int ME = RP::MEQN, MW = RP::MWAVES, NC = RP::NC, W = NT - 4;
-    constexpr int NI = (int)(sizeof(typename RP::Iface) / sizeof(double));
-    using Iface = typename RP::Iface;
-    static_assert(sizeof(Iface) % sizeof(double) == 0, "interface records are made of doubles");
-
-    const int t = threadIdx.x;
-    const int mx = a.L.mx, my = a.L.my;
-    const int pitch = a.L.pitch;
-    const long long plane = a.L.plane;
-    const int cp = strip * W + t;
-    const int cpl = min(cp, mx + 3);
-    const int Hb = min(a.H, my - rb);
-    const int R0 = rb, R1 = rb + Hb + 3;
-    const bool out_col = (t >= 2) && (t < W + 2) && (cp <= mx + 1);
-    const bool xcfl_col = (t >= 2) && (t <= W + 2) && (cp <= mx + 2);
-    const bool ycfl_col = (t >= 1) && (t <= W + 2) && (cp <= mx + 2);
-    const int tl = (t > 0) ? t - 1 : 0;
-    const int tr = (t < NT - 1) ? t + 1 : NT - 1;
-    // dt/dx, dt/dy: kernel parameters, or (EVO, the device time loop) the
-    // loop's record; a compile-time choice, so ordinary steps keep the
-    // parameters as operands of the FP64 instructions instead of registers
-    const double dtdx = EVO ? a.evo->dtdx : a.dtdx, dtdy = EVO ? a.evo->dtdy : a.dtdy;
-    const RPParams& P = a.rp;
-    const int order = (SPEC == SPEC_MC2) ? 2 : a.meth.order;
-    const int trans = (SPEC == SPEC_MC2) ? 2 : a.meth.transverse;
-    const bool tc = (order > 1) && (trans == 2);
-    const double* qo = a.qold + cpl;
-    double* qn = a.qnew + cpl;
-
-    constexpr int MA = AuxTraits<RP>::MAUX, MAD = MA > 0 ? MA : 1;
-    constexpr bool TAUX = AuxTraits<RP>::TRANSVERSE_AUX;
-    const double* ao = a.aux + cpl;
-    double pfa[MAD];
-#pragma unroll
-    for (int k = 0; k < MAD; ++k) pfa[k] = (MA > 0) ? __ldg(ao + k * plane + (long long)R0 * pitch) : 0.0;
-    const double* ko = CAPA ? a.capa + cpl : nullptr;
-    double pfk = CAPA ? __ldg(ko + (long long)R0 * pitch) : 1.0;
-
-    double pf[ME];
-    double accA[ME], accB[ME], accC[ME];  // rows R-2, R-1, R
-    Iface fY;                             // y-interface (R-2 | R-1)
-    double amY[ME], apY[ME], dY[MW];
-    unsigned long long n_it = 0, n_solve = 0, n_app = 0;
-#pragma unroll
-    for (int m = 0; m < ME; ++m) {
-        pf[m] = __ldg(qo + m * plane + (long long)R0 * pitch);
-        accA[m] = accB[m] = accC[m] = 0.0;
-        amY[m] = apY[m] = 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < MW; ++k) dY[k] = 0.0;
-    memset(&fY, 0, sizeof(fY));
-
-    int s2 = 0, s1 = 2, s0 = 1;  // ring slots of rows R, R-1, R-2
-    for (int R = R0; R <= R1; ++R) {
-        // ---- row R: prepare this column's cell, prefetch the next row ----
-        {
-            double q[ME], c[NC];
-#pragma unroll
-            for (int m = 0; m < ME; ++m) q[m] = pf[m];
-            if (R < R1) {
-#pragma unroll
-                for (int m = 0; m < ME; ++m) pf[m] = __ldg(qo + m * plane + (long long)(R + 1) * pitch);
-            }
-            double av[MAD];
-#pragma unroll
-            for (int k = 0; k < MAD; ++k) av[k] = pfa[k];
-            if (MA > 0 && R < R1) {
-#pragma unroll
-                for (int k = 0; k < MAD; ++k) pfa[k] = __ldg(ao + k * plane + (long long)(R + 1) * pitch);
-            }
-            AuxTraits<RP>::prep(q, av, P, c);
-#pragma unroll
-            for (int k = 0; k < NC; ++k) S.cell[s2][k][t] = c[k];
-            if constexpr (CAPA) {
-                S.icap[s2][t] = 1.0 / pfk;
-                if (R < R1) pfk = __ldg(ko + (long long)(R + 1) * pitch);
-            }
-        }
-        __syncthreads();  // S1: cells of row R and x-waves of row R-1 visible; previous exchange consumed
-
-        double xl0[ME], xl1[ME], xl2[ME], yr0[ME], yr1[ME];  // this row's increments for the neighbours
-#pragma unroll
-        for (int m = 0; m < ME; ++m) xl0[m] = xl1[m] = xl2[m] = yr0[m] = yr1[m] = 0.0;
-
-        // ---- x: finish the interface (cp-1 | cp) of row R-1 ----
-        if (R - 1 > R0 && R - 1 < R1) {  // rows R0+1 .. R1-1 carry x-interfaces
-            const int pb = (R - 1) & 1;
-            Iface fX;
-            double amX[ME], apX[ME];
-            {
-                double* fr = reinterpret_cast<double*>(&fX);
-#pragma unroll
-                for (int k = 0; k < NI; ++k) fr[k] = S.fx[k][t];
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    amX[m] = S.fx[NI + m][t];
-                    apX[m] = S.fx[NI + ME + m][t];
-                }
-            }
-            const double xdl = CAPA ? dtdx * S.icap[s1][tl] : dtdx, xdr = CAPA ? dtdx * S.icap[s1][t] : dtdx;
-            if (xcfl_col) cfl = fmax(cfl, CAPA ? iface_cfl2<RP, 1>(fX, P, xdl, xdr) : iface_cfl<RP, 1>(fX, P, dtdx));
-            double cq[ME];
-            if (order != 1) {
-                double dl[MW], dr[MW];
-#pragma unroll
-                for (int k = 0; k < MW; ++k) {
-                    double x = 0.0, y = 0.0;
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) {
-                        const double w = S.w[pb][k][m][t];
-                        x = x + S.w[pb][k][m][tl] * w;
-                        y = y + w * S.w[pb][k][m][tr];
-                    }
-                    dl[k] = x;
-                    dr[k] = y;
-                }
-                correction<RP, 1, SPEC>(fX, P, a.meth, CAPA ? 0.5 * (xdl + xdr) : dtdx, dl, dr, cq);
-            } else {
-#pragma unroll
-                for (int m = 0; m < ME; ++m) cq[m] = 0.0;
-            }
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                const double f = 0.5 * cq[m];
-                accB[m] = accB[m] - dtdx * (apX[m] - f);
-                xl1[m] = -dtdx * (amX[m] + f);
-            }
-            if (trans > 0) {
-                const double h = 0.5 * dtdx * dtdy;
-                const double hl = CAPA ? h * S.icap[s1][tl] : h, hr = CAPA ? h * S.icap[s1][t] : h;
-                double as2[ME], bm[ME], bp[ME];
-#pragma unroll
-                for (int m = 0; m < ME; ++m) as2[m] = tc ? amX[m] + cq[m] : amX[m];
-                if constexpr (TAUX) {  // cell (cp-1, R-1) between rows R-2 and R
-                    double cm[NC], c0[NC], cu[NC];
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) {
-                        cm[k] = S.cell[s0][k][tl];
-                        c0[k] = S.cell[s1][k][tl];
-                        cu[k] = S.cell[s2][k][tl];
-                    }
-                    RP::template rpt2_aux<1>(as2, cm, c0, cu, bm, bp);
-                } else {
-                    RP::template rpt2<1>(fX, P, as2, bm, bp);  // imp = 1 -> column cp-1
-                }
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    xl1[m] = xl1[m] + hl * (bp[m] - bm[m]);
-                    xl0[m] = hl * bm[m];
-                    xl2[m] = -hl * bp[m];
-                }
-#pragma unroll
-                for (int m = 0; m < ME; ++m) as2[m] = tc ? apX[m] - cq[m] : apX[m];
-                if constexpr (TAUX) {  // cell (cp, R-1)
-                    double cm[NC], c0[NC], cu[NC];
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) {
-                        cm[k] = S.cell[s0][k][t];
-                        c0[k] = S.cell[s1][k][t];
-                        cu[k] = S.cell[s2][k][t];
-                    }
-                    RP::template rpt2_aux<1>(as2, cm, c0, cu, bm, bp);
-                } else {
-                    RP::template rpt2<1>(fX, P, as2, bm, bp);  // imp = 2 -> column cp
-                }
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    accB[m] = accB[m] + hr * (bp[m] - bm[m]);
-                    accA[m] = accA[m] + hr * bm[m];
-                    accC[m] = accC[m] - hr * bp[m];
-                }
-            }
-        }
-
-        // ---- y: solve (R-1 | R), finish (R-2 | R-1) ----
-        if (R > R0) {
-            double cB[NC], cA[NC];
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                cB[k] = S.cell[s1][k][t];
-                cA[k] = S.cell[s2][k][t];
-            }
-            Iface fN;
-            double amN[ME], apN[ME];
-            double gy = 0.0;
-            if (GuessTraits<RP>::USES && a.guess) gy = a.guess[plane + (long long)R * pitch + cpl];
-            GuessTraits<RP>::template solve<2>(cB, cA, P, gy, fN, amN, apN);
-            if (GuessTraits<RP>::USES && cp <= mx + 3) {
-                n_it += GuessTraits<RP>::count(fN);
-                n_app += GuessTraits<RP>::count_applied(fN);
-                n_solve += 1;
-            }
-            double dn[MW];
-            {
-                double wY[MW][ME], wN[MW][ME];
-                RP::template waves<2>(fY, P, wY);
-                RP::template waves<2>(fN, P, wN);
-#pragma unroll
-                for (int k = 0; k < MW; ++k) {
-                    double d = 0.0;
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) d = d + wY[k][m] * wN[k][m];
-                    dn[k] = d;
-                }
-            }
-            if (R >= R0 + 3) {
-                const double ydl = CAPA ? dtdy * S.icap[s0][t] : dtdy, ydr = CAPA ? dtdy * S.icap[s1][t] : dtdy;
-                if (ycfl_col)
-                    cfl = fmax(cfl, CAPA ? iface_cfl2<RP, 2>(fY, P, ydl, ydr) : iface_cfl<RP, 2>(fY, P, dtdy));
-                double cq[ME];
-                if (order != 1) {
-                    correction<RP, 2, SPEC>(fY, P, a.meth, CAPA ? 0.5 * (ydl + ydr) : dtdy, dY, dn, cq);
-                } else {
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) cq[m] = 0.0;
-                }
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    const double f = 0.5 * cq[m];
-                    accA[m] = accA[m] - dtdy * (amY[m] + f);
-                    accB[m] = accB[m] - dtdy * (apY[m] - f);
-                }
-                if (trans > 0) {
-                    const double h = 0.5 * dtdy * dtdx;
-                    const double hl = CAPA ? h * S.icap[s0][t] : h, hr = CAPA ? h * S.icap[s1][t] : h;
-                    double as2[ME], bm[ME], bp[ME];
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) as2[m] = tc ? amY[m] + cq[m] : amY[m];
-                    if constexpr (TAUX) {  // cell (cp, R-2) between columns cp-1 and cp+1
-                        double cm[NC], c0[NC], cu[NC];
-#pragma unroll
-                        for (int k = 0; k < NC; ++k) {
-                            cm[k] = S.cell[s0][k][tl];
-                            c0[k] = S.cell[s0][k][t];
-                            cu[k] = S.cell[s0][k][tr];
-                        }
-                        RP::template rpt2_aux<2>(as2, cm, c0, cu, bm, bp);
-                    } else {
-                        RP::template rpt2<2>(fY, P, as2, bm, bp);  // imp = 1 -> row R-2
-                    }
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) {
-                        accA[m] = accA[m] + hl * (bp[m] - bm[m]);
-                        xl0[m] = xl0[m] + hl * bm[m];
-                        yr0[m] = -hl * bp[m];
-                    }
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) as2[m] = tc ? apY[m] - cq[m] : apY[m];
-                    if constexpr (TAUX) {  // cell (cp, R-1)
-                        double cm[NC], c0[NC], cu[NC];
-#pragma unroll
-                        for (int k = 0; k < NC; ++k) {
-                            cm[k] = S.cell[s1][k][tl];
-                            c0[k] = S.cell[s1][k][t];
-                            cu[k] = S.cell[s1][k][tr];
-                        }
-                        RP::template rpt2_aux<2>(as2, cm, c0, cu, bm, bp);
-                    } else {
-                        RP::template rpt2<2>(fY, P, as2, bm, bp);  // imp = 2 -> row R-1
-                    }
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) {
-                        accB[m] = accB[m] + hr * (bp[m] - bm[m]);
-                        xl1[m] = xl1[m] + hr * bm[m];
-                        yr1[m] = -hr * bp[m];
-                    }
-                }
-            }
-            fY = fN;
-#pragma unroll
-            for (int m = 0; m < ME; ++m) { amY[m] = amN[m]; apY[m] = apN[m]; }
-#pragma unroll
-            for (int k = 0; k < MW; ++k) dY[k] = dn[k];
-        }
-
-        // ---- x: solve the interface (cp-1 | cp) of row R, keep it for the next row ----
-        if (R > R0 && R < R1) {
-            double cL[NC], cR[NC];
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                cL[k] = S.cell[s2][k][tl];
-                cR[k] = S.cell[s2][k][t];
-            }
-            Iface fX;
-            double amX[ME], apX[ME];
-            double gx = 0.0;
-            if (GuessTraits<RP>::USES && a.guess) gx = a.guess[(long long)R * pitch + cpl];
-            GuessTraits<RP>::template solve<1>(cL, cR, P, gx, fX, amX, apX);
-            if (GuessTraits<RP>::USES && cp <= mx + 3 && t > 0) {
-                n_it += GuessTraits<RP>::count(fX);
-                n_app += GuessTraits<RP>::count_applied(fX);
-                n_solve += 1;
-            }
-            double wX[MW][ME];
-            RP::template waves<1>(fX, P, wX);
-            const int pb = R & 1;
-#pragma unroll
-            for (int k = 0; k < MW; ++k)
-#pragma unroll
-                for (int m = 0; m < ME; ++m) S.w[pb][k][m][t] = wX[k][m];
-            const double* fr = reinterpret_cast<const double*>(&fX);
-#pragma unroll
-            for (int k = 0; k < NI; ++k) S.fx[k][t] = fr[k];
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                S.fx[NI + m][t] = amX[m];
-                S.fx[NI + ME + m][t] = apX[m];
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < ME; ++m) {
-            S.xl[0][m][t] = xl0[m];
-            S.xl[1][m][t] = xl1[m];
-            S.xl[2][m][t] = xl2[m];
-            S.yr[0][m][t] = yr0[m];
-            S.yr[1][m][t] = yr1[m];
-        }
-        __syncthreads();  // S2: neighbour increments (and this row's x-waves) visible
-#pragma unroll
-        for (int m = 0; m < ME; ++m) {
-            accA[m] = accA[m] + S.xl[0][m][tr] + S.yr[0][m][tl];
-            accB[m] = accB[m] + S.xl[1][m][tr] + S.yr[1][m][tl];
-            accC[m] = accC[m] + S.xl[2][m][tr];
-        }
-
-        // ---- row R-2 is complete ----
-        if (R >= R0 + 4 && out_col) {
-            double v[ME];
-            const double ik = CAPA ? S.icap[s0][t] : 1.0;
-#pragma unroll
-            for (int m = 0; m < ME; ++m) v[m] = CAPA ? S.cell[s0][m][t] + ik * accA[m] : S.cell[s0][m][t] + accA[m];
-#pragma unroll
-            for (int m = 0; m < ME; ++m) qn[m * plane + (long long)(R - 2) * pitch] = v[m];
-            if (!all_finite<ME>(v)) atomicOr(a.status, 1);
-        }
-#pragma unroll
-        for (int m = 0; m < ME; ++m) {
-            accA[m] = accB[m];
-            accB[m] = accC[m];
-            accC[m] = 0.0;
-        }
-        const int tmp = s0;
-        s0 = s1;
-        s1 = s2;
-        s2 = tmp;
-    }
-    if (GuessTraits<RP>::USES && a.counters) counter_commit(a.counters, n_it, n_solve, n_app);
-}
-
-template <class RP, int NT, int MINB, int SPEC, bool CAPA = false, bool EVO = false>
-__global__ void __launch_bounds__(NT, MINB) k_step_unsplit2(const StepArgs a) {
-    if (EVO && a.evo->done) return;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    UnsplitSmem2<RP, NT, CAPA>& S = *reinterpret_cast<UnsplitSmem2<RP, NT, CAPA>*>(smem_raw);
-    const int tile = tile_index(a);
-    long long t0 = 0;
-    if (a.tile_cost && threadIdx.x == 0) t0 = clock64();
-    double cfl = 0.0;
-    unsplit_tile2<RP, NT, SPEC, CAPA, EVO>(a, tile % a.nstrips, (tile / a.nstrips) * a.H, S, cfl);
-    cfl_commit(cfl, S.red, a.cfl_bits);
-    if (a.tile_cost && threadIdx.x == 0) {
-        const long long c = clock64() - t0;
-        a.tile_cost[tile] = (unsigned int)(c < 0 ? 0 : (c > 0xffffffffll ? 0xffffffffll : c));
-    }
-}
-
-// ---------------------------------------------------------------------------
-// The direction-split tile: two threads per column.  The CTA has 2*NT
-// threads; the first NT (the Y warps) own the y-interfaces of their column
-// and the second NT (the X warps) its x-interfaces, so each thread carries
-// half the live state of unsplit_tile and twice as many warps fit on an SM
-// (16 instead of 8 for Euler), which is what the FP64 pipe of a latency-bound
-// step needs.  The two warp groups meet only through named barriers used by
-// row parity, so the x work of a row overlaps the y work of the same row:
-//   Y, row R: [wait EMPTY(R-1)] prepare the column's cell of row R into a
-//      4-row ring, prefetch row R+1, [arrive CELLS(R)]; solve (R-1 | R);
-//      finish (R-2 | R-1) (limiter with the waves below and above,
-//      correction, two transverse solves); [Y] exchange with the neighbour
-//      columns [Y]; write row R-3 = q + (its y total + the X group's total);
-//      after the last row, [wait EMPTY(R1)] and write row R1-2.
-//   X, row R: [wait CELLS(R)] solve (cp-1 | cp) of row R, store its waves
-//      [X]; gather the neighbour's increments of row R-1, publish its total of
-//      row R-2; finish row R (limiter with the neighbours' waves, correction,
-//      two transverse solves), publish column cp-1's increments [X];
-//      [arrive EMPTY(R)].
-// CELLS(R): row R's cells are in the ring.  EMPTY(R): the X group is done
-// with row R (so the ring slot that row R+1 reuses, rows R-3's, and the
-// total buffer Y reads next are free).  Both are pairs of barriers used by
-// row parity, each with all 2*NT threads; [X] and [Y] are the groups' own
-// barriers.  Every arrival has its wait: Y arrives CELLS on every row and X
-// waits on every row; X arrives EMPTY on every row and Y waits on rows
-// R0+1..R1 and once after the loop.  The y-interface being finished, its
-// fluctuations and its dot products wait in shared memory (per column,
-// touched only by that column's Y thread).  The increments are the same
-// terms as in unsplit_tile; only the order of the per-cell sum differs (the
-// x and y parts are summed apart and then added).  Solvers without aux data
-// or guesses, no capacity form.
-// ---------------------------------------------------------------------------
-template <class RP, int NT>
-struct UnsplitSmemWS {
-    static constexpr int ME = RP::MEQN, MW = RP::MWAVES, NC = RP::NC;
-    static constexpr int NF = (int)(sizeof(typename RP::Iface) / sizeof(double));
-    double cell[4][NC][NT];          // prepared cells, row R in slot R & 3 (Y writes)
-    double w[MW][ME][NT];            // unlimited x-waves of the current row (X)
-    double xl[3][ME][NT];            // X -> column cp-1: rows R-1, R, R+1
-    double yl[2][ME][NT];            // Y -> column cp-1: rows R-2, R-1
-    double yr[2][ME][NT];            // Y -> column cp+1: rows R-2, R-1
-    double xs[2][ME][NT];            // X's total of row R-2, by row parity (X -> Y)
-    double fy[NF][NT];               // Y: the y-interface being finished, (R-2 | R-1)
-    double amy[ME][NT], apy[ME][NT];  // its fluctuations
-    double dy[MW][NT];               // its waves' dot products with the waves below it
-    double red[2 * NT / 32];
-};
-
-// named barriers of the direction-split tile (0 is __syncthreads)
-enum { NB_X = 1, NB_Y = 2, NB_CELLS = 3, NB_EMPTY = 5 };
-
-template <int ID, int N>
-__device__ __forceinline__ void nb_sync() {
-    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
-}
-template <int ID, int N>
-__device__ __forceinline__ void nb_arrive() {
-    asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(N) : "memory");
-}
-// the barrier of a pair chosen by row parity (compile-time ids)
-template <int ID, int N>
-__device__ __forceinline__ void nb_sync_parity(int R) {
-    if (R & 1) nb_sync<ID + 1, N>();
-    else nb_sync<ID, N>();
-}
-template <int ID, int N>
-__device__ __forceinline__ void nb_arrive_parity(int R) {
-    if (R & 1) nb_arrive<ID + 1, N>();
-    else nb_arrive<ID, N>();
-}
-
-template <class RP, int NT, int SPEC = SPEC_ANY, bool EVO = false, int REG_Y = 0, int REG_X = 0>
-__device__ __forceinline__ void unsplit_tile_ws(const StepArgs& a, int strip, int rb, UnsplitSmemWS<RP, NT>& S,
-                                                double& cfl) {
-    constexpr int ME = RP::MEQN, MW = RP::MWAVES, NC = RP::NC, W = NT - 4;
-    constexpr int NF = UnsplitSmemWS<RP, NT>::NF;
-    using Iface = typename RP::Iface;
-    static_assert(AuxTraits<RP>::MAUX == 0 && !GuessTraits<RP>::USES, "direction-split tile: no aux, no guess");
-
-    const bool yrole = threadIdx.x < NT;
-    const int t = yrole ? threadIdx.x : threadIdx.x - NT;
-    const int mx = a.L.mx, my = a.L.my;
-    const int pitch = a.L.pitch;
-    const long long plane = a.L.plane;
-    const int cp = strip * W + t;
-    const int cpl = min(cp, mx + 3);
-    const int Hb = min(a.H, my - rb);
-    const int R0 = rb, R1 = rb + Hb + 3;
-    const bool out_col = (t >= 2) && (t < W + 2) && (cp <= mx + 1);
-    const bool xcfl_col = (t >= 2) && (t <= W + 2) && (cp <= mx + 2);
-    const bool ycfl_col = (t >= 1) && (t <= W + 2) && (cp <= mx + 2);
-    const int tl = (t > 0) ? t - 1 : 0;
-    const int tr = (t < NT - 1) ? t + 1 : NT - 1;
-    const double dtdx = EVO ? a.evo->dtdx : a.dtdx, dtdy = EVO ? a.evo->dtdy : a.dtdy;
-    const RPParams& P = a.rp;
-    const int order = (SPEC == SPEC_MC2) ? 2 : a.meth.order;
-    const int trans = (SPEC == SPEC_MC2) ? 2 : a.meth.transverse;
-    const bool tc = (order > 1) && (trans == 2);
-    constexpr bool ZS = SkipTraits<RP>::OK;
-    const bool zs = ZS && (SPEC != SPEC_ANY || a.meth.fwave == 0);
-    constexpr int N2 = 2 * NT;
-
-    if (yrole) {
-        // ================= Y warps =================
-        if (REG_Y > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_Y));
-        const double* qo = a.qold + cpl;
-        double* qn = a.qnew + cpl;
-        double pf[ME], yA[ME], yB[ME], yC[ME];  // prefetched row; increments of rows R-2, R-1; total of R-3
-#pragma unroll
-        for (int m = 0; m < ME; ++m) {
-            pf[m] = __ldg(qo + m * plane + (long long)R0 * pitch);
-            yA[m] = yB[m] = yC[m] = 0.0;
-        }
-        bool zY = false;
-        for (int R = R0; R <= R1; ++R) {
-            const int s2 = R & 3, s1 = (R - 1) & 3;
-            if (R >= R0 + 1) nb_sync_parity<NB_EMPTY, N2>(R - 1);  // X done with row R-1: the slot of R-4 is free
-            {
-                double q[ME], c[NC];
-#pragma unroll
-                for (int m = 0; m < ME; ++m) q[m] = pf[m];
-                if (R < R1) {
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) pf[m] = __ldg(qo + m * plane + (long long)(R + 1) * pitch);
-                }
-                RP::prepare(q, P, c);
-#pragma unroll
-                for (int k = 0; k < NC; ++k) S.cell[s2][k][t] = c[k];
-            }
-            nb_arrive_parity<NB_CELLS, N2>(R);  // row R prepared
-            double ylB[ME], ylA[ME], yrB[ME], yrA[ME];
-#pragma unroll
-            for (int m = 0; m < ME; ++m) ylB[m] = ylA[m] = yrB[m] = yrA[m] = 0.0;
-            if (R > R0) {
-                double cB[NC], cA[NC];
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    cB[k] = S.cell[s1][k][t];
-                    cA[k] = S.cell[s2][k][t];
-                }
-                Iface fN, fY;
-                double amN[ME], apN[ME], dn[MW];
-                const bool zN = zs && __all_sync(0xffffffffu, same_q<ME, NC>(cB, cA));
-                {
-                    double* fp = reinterpret_cast<double*>(&fY);
-#pragma unroll
-                    for (int k = 0; k < NF; ++k) fp[k] = S.fy[k][t];
-                }
-                if (ZS && zN) {
-                    SkipTraits<RP>::template zero_iface<2>(cB, cA, P, fN);
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) amN[m] = apN[m] = 0.0;
-#pragma unroll
-                    for (int k = 0; k < MW; ++k) dn[k] = 0.0;
-                } else {
-                    RP::template solve<2>(cB, cA, P, fN, amN, apN);
-                    double wY[MW][ME], wN[MW][ME];
-                    RP::template waves<2>(fY, P, wY);
-                    RP::template waves<2>(fN, P, wN);
-#pragma unroll
-                    for (int k = 0; k < MW; ++k) {
-                        double d = 0.0;
-#pragma unroll
-                        for (int m = 0; m < ME; ++m) d = d + wY[k][m] * wN[k][m];
-                        dn[k] = d;
-                    }
-                }
-                if (R >= R0 + 3) {
-                    if (ycfl_col) cfl = fmax(cfl, iface_cfl<RP, 2>(fY, P, dtdy));
-                    if (!(ZS && zY)) {
-                        double amY[ME], apY[ME], dY[MW], cq[ME];
-#pragma unroll
-                        for (int m = 0; m < ME; ++m) {
-                            amY[m] = S.amy[m][t];
-                            apY[m] = S.apy[m][t];
-                        }
-#pragma unroll
-                        for (int k = 0; k < MW; ++k) dY[k] = S.dy[k][t];
-                        if (order != 1) {
-                            correction<RP, 2, SPEC>(fY, P, a.meth, dtdy, dY, dn, cq);
-                        } else {
-#pragma unroll
-                            for (int m = 0; m < ME; ++m) cq[m] = 0.0;
-                        }
-#pragma unroll
-                        for (int m = 0; m < ME; ++m) {
-                            const double f = 0.5 * cq[m];
-                            yA[m] = yA[m] - dtdy * (amY[m] + f);
-                            yB[m] = yB[m] - dtdy * (apY[m] - f);
-                        }
-                        if (trans > 0) {
-                            const double h = 0.5 * dtdy * dtdx;
-                            double as2[ME], bm[ME], bp[ME];
-#pragma unroll
-                            for (int m = 0; m < ME; ++m) as2[m] = tc ? amY[m] + cq[m] : amY[m];
-                            RP::template rpt2<2>(fY, P, as2, bm, bp);  // imp = 1 -> row R-2
-#pragma unroll
-                            for (int m = 0; m < ME; ++m) {
-                                yA[m] = yA[m] + h * (bp[m] - bm[m]);
-                                ylB[m] = h * bm[m];
-                                yrB[m] = -h * bp[m];
-                            }
-#pragma unroll
-                            for (int m = 0; m < ME; ++m) as2[m] = tc ? apY[m] - cq[m] : apY[m];
-                            RP::template rpt2<2>(fY, P, as2, bm, bp);  // imp = 2 -> row R-1
-#pragma unroll
-                            for (int m = 0; m < ME; ++m) {
-                                yB[m] = yB[m] + h * (bp[m] - bm[m]);
-                                ylA[m] = h * bm[m];
-                                yrA[m] = -h * bp[m];
-                            }
-                        }
-                    }
-                }
-                {
-                    const double* fp = reinterpret_cast<const double*>(&fN);
-#pragma unroll
-                    for (int k = 0; k < NF; ++k) S.fy[k][t] = fp[k];
-                }
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    S.amy[m][t] = amN[m];
-                    S.apy[m][t] = apN[m];
-                }
-#pragma unroll
-                for (int k = 0; k < MW; ++k) S.dy[k][t] = dn[k];
-                zY = zN;
-            } else {
-                // the first row: an empty record below it (zero waves, zero dots)
-#pragma unroll
-                for (int k = 0; k < NF; ++k) S.fy[k][t] = 0.0;
-            }
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                S.yl[0][m][t] = ylB[m];
-                S.yl[1][m][t] = ylA[m];
-                S.yr[0][m][t] = yrB[m];
-                S.yr[1][m][t] = yrA[m];
-            }
-            nb_sync<NB_Y, NT>();  // the Y warps' neighbour increments visible
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                yA[m] = yA[m] + S.yl[0][m][tr] + S.yr[0][m][tl];
-                yB[m] = yB[m] + S.yl[1][m][tr] + S.yr[1][m][tl];
-            }
-            nb_sync<NB_Y, NT>();  // every read of the exchange done before the next row's writes
-            if (R >= R0 + 5 && out_col) {  // row R-3: both totals complete (X's since its row R-1)
-                double v[ME];
-#pragma unroll
-                for (int m = 0; m < ME; ++m) v[m] = S.cell[(R - 3) & 3][m][t] + (yC[m] + S.xs[(R - 3) & 1][m][t]);
-#pragma unroll
-                for (int m = 0; m < ME; ++m) qn[m * plane + (long long)(R - 3) * pitch] = v[m];
-                if (!all_finite<ME>(v)) atomicOr(a.status, 1);
-            }
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                yC[m] = yA[m];  // row R-2 complete on the y side
-                yA[m] = yB[m];
-                yB[m] = 0.0;
-            }
-        }
-        nb_sync_parity<NB_EMPTY, N2>(R1);  // X done with the last row: its total of row R1-2
-        if (R1 >= R0 + 4 && out_col) {
-            double v[ME];
-#pragma unroll
-            for (int m = 0; m < ME; ++m) v[m] = S.cell[(R1 - 2) & 3][m][t] + (yC[m] + S.xs[(R1 - 2) & 1][m][t]);
-#pragma unroll
-            for (int m = 0; m < ME; ++m) qn[m * plane + (long long)(R1 - 2) * pitch] = v[m];
-            if (!all_finite<ME>(v)) atomicOr(a.status, 1);
-        }
-    } else {
-        // ================= X warps =================
-        if (REG_X > 0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_X));
-        double x0[ME], x1[ME], x2[ME];  // increments of rows R-2, R-1, R (this column)
-#pragma unroll
-        for (int m = 0; m < ME; ++m) x0[m] = x1[m] = x2[m] = 0.0;
-        for (int R = R0; R <= R1; ++R) {
-            const int s2 = R & 3;
-            nb_sync_parity<NB_CELLS, N2>(R);  // row R prepared
-            Iface fX;
-            double amX[ME], apX[ME];
-            bool zX;
-            const bool xrow = (R > R0) && (R < R1);
-            {
-                double cL[NC], cR[NC];
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    cL[k] = S.cell[s2][k][tl];
-                    cR[k] = S.cell[s2][k][t];
-                }
-                // (the first and last rows' x-interfaces are never finished: no solve)
-                zX = ZS && (!xrow || (zs && __all_sync(0xffffffffu, same_q<ME, NC>(cL, cR))));
-                if (ZS && zX) {
-                    SkipTraits<RP>::template zero_iface<1>(cL, cR, P, fX);
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) amX[m] = apX[m] = 0.0;
-#pragma unroll
-                    for (int k = 0; k < MW; ++k)
-#pragma unroll
-                        for (int m = 0; m < ME; ++m) S.w[k][m][t] = 0.0;
-                } else {
-                    RP::template solve<1>(cL, cR, P, fX, amX, apX);
-                    double wX[MW][ME];
-                    RP::template waves<1>(fX, P, wX);
-#pragma unroll
-                    for (int k = 0; k < MW; ++k)
-#pragma unroll
-                        for (int m = 0; m < ME; ++m) S.w[k][m][t] = wX[k][m];
-                }
-            }
-            nb_sync<NB_X, NT>();  // x-waves of row R and column cp-1's increments of row R-1 visible
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                x0[m] = x0[m] + S.xl[0][m][tr];  // rows R-2, R-1, R from the neighbour's row R-1
-                x1[m] = x1[m] + S.xl[1][m][tr];
-                x2[m] = x2[m] + S.xl[2][m][tr];
-                S.xs[R & 1][m][t] = x0[m];  // row R-2 complete on the x side
-            }
-            double x3[ME], xbL[ME], xcL[ME], xaL[ME];
-#pragma unroll
-            for (int m = 0; m < ME; ++m) x3[m] = xbL[m] = xcL[m] = xaL[m] = 0.0;
-            if (xrow && xcfl_col) cfl = fmax(cfl, iface_cfl<RP, 1>(fX, P, dtdx));
-            if (xrow && !(ZS && zX)) {
-                double cq[ME];
-                if (order != 1) {
-                    double dl[MW], dr[MW];
-#pragma unroll
-                    for (int k = 0; k < MW; ++k) {
-                        double x = 0.0, y = 0.0;
-#pragma unroll
-                        for (int m = 0; m < ME; ++m) {
-                            const double w = S.w[k][m][t];
-                            x = x + S.w[k][m][tl] * w;
-                            y = y + w * S.w[k][m][tr];
-                        }
-                        dl[k] = x;
-                        dr[k] = y;
-                    }
-                    correction<RP, 1, SPEC>(fX, P, a.meth, dtdx, dl, dr, cq);
-                } else {
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) cq[m] = 0.0;
-                }
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    const double f = 0.5 * cq[m];
-                    x2[m] = x2[m] - dtdx * (apX[m] - f);
-                    xcL[m] = -dtdx * (amX[m] + f);
-                }
-                if (trans > 0) {
-                    const double h = 0.5 * dtdx * dtdy;
-                    double as2[ME], bm[ME], bp[ME];
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) as2[m] = tc ? amX[m] + cq[m] : amX[m];
-                    RP::template rpt2<1>(fX, P, as2, bm, bp);  // imp = 1 -> column cp-1
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) {
-                        xcL[m] = xcL[m] + h * (bp[m] - bm[m]);
-                        xbL[m] = h * bm[m];
-                        xaL[m] = -h * bp[m];
-                    }
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) as2[m] = tc ? apX[m] - cq[m] : apX[m];
-                    RP::template rpt2<1>(fX, P, as2, bm, bp);  // imp = 2 -> column cp
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) {
-                        x2[m] = x2[m] + h * (bp[m] - bm[m]);
-                        x1[m] = x1[m] + h * bm[m];
-                        x3[m] = x3[m] - h * bp[m];
-                    }
-                }
-            }
-            nb_sync<NB_X, NT>();  // every read of the waves and of the exchange slots done
-#pragma unroll
-            for (int m = 0; m < ME; ++m) {
-                S.xl[0][m][t] = xbL[m];
-                S.xl[1][m][t] = xcL[m];
-                S.xl[2][m][t] = xaL[m];
-                x0[m] = x1[m];
-                x1[m] = x2[m];
-                x2[m] = x3[m];
-            }
-            nb_arrive_parity<NB_EMPTY, N2>(R);  // done with row R; its total of row R-2 published
-        }
-    }
-}
-
-// Grid: 1D over the tiles as k_step_unsplit, 2*NT threads per CTA.
-template <class RP, int NT, int MINB, int SPEC, bool EVO = false, int REG_Y = 0, int REG_X = 0>
-__global__ void __launch_bounds__(2 * NT, MINB) k_step_unsplit_ws(const StepArgs a) {
-    if (EVO && a.evo->done) return;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    UnsplitSmemWS<RP, NT>& S = *reinterpret_cast<UnsplitSmemWS<RP, NT>*>(smem_raw);
-    const int tile = tile_index(a);
-    long long t0 = 0;
-    if (a.tile_cost && threadIdx.x == 0) t0 = clock64();
-    double cfl = 0.0;
-    unsplit_tile_ws<RP, NT, SPEC, EVO, REG_Y, REG_X>(a, tile % a.nstrips, (tile / a.nstrips) * a.H, S, cfl);
-    cfl_commit(cfl, S.red, a.cfl_bits);
-    if (a.tile_cost && threadIdx.x == 0) {
-        const long long c = clock64() - t0;
-        a.tile_cost[tile] = (unsigned int)(c < 0 ? 0 : (c > 0xffffffffll ? 0xffffffffll : c));
-    }
 }
 
 // The same kernel with its rows staged by TMA from the tensor map of qold.
@@ -1695,7 +916,7 @@ struct SplitXSmem {
     static constexpr int ME = RP::MEQN, MW = RP::MWAVES, NC = RP::NC;
     double cell[2][NC][NT];
     double icap[2][NT];  // 1 / kappa (1 without a capacity function)
-    double w[MW][ME][NT];
+    double w[Lim<RP>::N][NT];
     double xl[ME][NT];
     double red[NT / 32];
 };
@@ -1761,19 +982,13 @@ __global__ void __launch_bounds__(NT) k_split_x(const StepArgs a) {
                 SkipTraits<RP>::template zero_iface<1>(cL, cR, P, fX);
 #pragma unroll
                 for (int m = 0; m < ME; ++m) amX[m] = apX[m] = 0.0;
-#pragma unroll
-                for (int k = 0; k < MW; ++k)
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) S.w[k][m][t] = 0.0;
             } else {
                 RP::template solve<1>(cL, cR, P, fX, amX, apX);
-                double wX[MW][ME];
-                RP::template waves<1>(fX, P, wX);
-#pragma unroll
-                for (int k = 0; k < MW; ++k)
-#pragma unroll
-                    for (int m = 0; m < ME; ++m) S.w[k][m][t] = wX[k][m];
             }
+            double rX[Lim<RP>::N];
+            Lim<RP>::template rec<1>(fX, P, rX);
+#pragma unroll
+            for (int k = 0; k < Lim<RP>::N; ++k) S.w[k][t] = rX[k];
         }
         __syncthreads();
         // dt/(dx kappa) left and right of the interface (both dtdx without capacity)
@@ -1781,20 +996,11 @@ __global__ void __launch_bounds__(NT) k_split_x(const StepArgs a) {
         if (xcfl_col) cfl = fmax(cfl, iface_cfl2<RP, 1>(fX, P, xdl, xdr));
         double cq[ME];
         if (!(ZS && zX) && ((SPEC != SPEC_ANY) || a.meth.order != 1)) {
-            double dl[MW], dr[MW];
-#pragma unroll
-            for (int k = 0; k < MW; ++k) {
-                double x = 0.0, y = 0.0;
-#pragma unroll
-                for (int m = 0; m < ME; ++m) {
-                    const double w = S.w[k][m][t];
-                    x = x + S.w[k][m][tl] * w;
-                    y = y + w * S.w[k][m][tr];
-                }
-                dl[k] = x;
-                dr[k] = y;
-            }
-            correction<RP, 1, SPEC>(fX, P, a.meth, 0.5 * (xdl + xdr), dl, dr, cq);
+            double rX[Lim<RP>::N], sX[MW], num[MW];
+            Lim<RP>::template rec<1>(fX, P, rX);
+            RP::template speeds<1>(fX, P, sX);
+            Lim<RP>::up(rX, sX, [&](int j, bool left) { return S.w[j][left ? tl : tr]; }, num);
+            correction<RP, 1, SPEC>(fX, P, a.meth, 0.5 * (xdl + xdr), rX, sX, num, cq);
         } else {
 #pragma unroll
             for (int m = 0; m < ME; ++m) cq[m] = 0.0;
@@ -1884,25 +1090,24 @@ __global__ void __launch_bounds__(NT) k_split_y(const StepArgs a) {
         const double ic2 = ko ? 1.0 / __ldg(ko + (long long)R * pitch) : 1.0;
         Iface fN;
         double amN[ME], apN[ME];
-        double dn[MW];
+        double dn[MW], da[MW];  // limiter numerators (see unsplit_tile)
         const bool zN = ZS && zs && __all_sync(0xffffffffu, same_q<ME, NC>(cB, cA));
         if (ZS && zN) {
             SkipTraits<RP>::template zero_iface<2>(cB, cA, P, fN);
 #pragma unroll
             for (int m = 0; m < ME; ++m) amN[m] = apN[m] = 0.0;
 #pragma unroll
-            for (int k = 0; k < MW; ++k) dn[k] = 0.0;
+            for (int k = 0; k < MW; ++k) dn[k] = da[k] = 0.0;
         } else {
             RP::template solve<2>(cB, cA, P, fN, amN, apN);
-            double wY[MW][ME], wN[MW][ME];
-            RP::template waves<2>(fY, P, wY);
-            RP::template waves<2>(fN, P, wN);
+            double rY[Lim<RP>::N], rN[Lim<RP>::N], X[MW];
+            Lim<RP>::template rec<2>(fY, P, rY);
+            Lim<RP>::template rec<2>(fN, P, rN);
+            Lim<RP>::cross(rY, rN, X);
 #pragma unroll
             for (int k = 0; k < MW; ++k) {
-                double d = 0.0;
-#pragma unroll
-                for (int m = 0; m < ME; ++m) d = d + wY[k][m] * wN[k][m];
-                dn[k] = d;
+                dn[k] = Lim<RP>::amp(rY, k) * X[k];
+                da[k] = Lim<RP>::amp(rN, k) * X[k];
             }
         }
         // acc0 <-> row R-2, acc1 <-> row R-1
@@ -1914,7 +1119,12 @@ __global__ void __launch_bounds__(NT) k_split_y(const StepArgs a) {
             const double ydl = dtdy * ic0, ydr = dtdy * ic1;
             double cq[ME];
             if ((SPEC != SPEC_ANY) || a.meth.order != 1) {
-                correction<RP, 2, SPEC>(fY, P, a.meth, 0.5 * (ydl + ydr), dY, dn, cq);
+                double rY[Lim<RP>::N], sY[MW], num[MW];
+                Lim<RP>::template rec<2>(fY, P, rY);
+                RP::template speeds<2>(fY, P, sY);
+#pragma unroll
+                for (int k = 0; k < MW; ++k) num[k] = (sY[k] > 0.0) ? dY[k] : da[k];
+                correction<RP, 2, SPEC>(fY, P, a.meth, 0.5 * (ydl + ydr), rY, sY, num, cq);
             } else {
 #pragma unroll
                 for (int m = 0; m < ME; ++m) cq[m] = 0.0;

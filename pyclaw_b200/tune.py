@@ -12,7 +12,7 @@ import statistics
 from . import _lib
 
 ROWS = (2, 4, 8, 12, 14, 16, 18, 20, 24, 28, 32, 48, 64)
-VARIANTS = (0, 1, 2, 3, 4, 8)
+VARIANTS = (0, 1, 2, 3)
 _cache = {}
 
 

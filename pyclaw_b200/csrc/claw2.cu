@@ -564,7 +564,8 @@ int host_step(int maxm, int meqn, int mwaves, int maux, int mbc, int mx, int my,
 struct claw2_mlp {
     int device = 0;
     float* P = nullptr;      // parameters (FP32)
-    float* G = nullptr;      // gradient accumulator
+    float* G = nullptr;      // gradient (claw2_mlp_gradient)
+    float* part = nullptr;   // k_train_grad's partial sums, train_rows() rows
     float* M1 = nullptr;     // Adam moments
     float* M2 = nullptr;
     float* loss = nullptr;
@@ -594,6 +595,21 @@ int mlp_repack(claw2_mlp* m) {
     mlp_pack_tc(h.data(), ti);
     CUDA_TRY(cudaMemcpy(m->tc, &ti, sizeof ti, cudaMemcpyHostToDevice));
     return CLAW2_OK;
+}
+
+// Rows of a network's partial-sum array: four CTAs of k_train_grad per SM.
+int train_cap(int device) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
+    return 4 * n;
+}
+
+// One minibatch: gradient sums, then Adam (grad == nullptr) or the gradient.
+void mlp_batch_launch(claw2_mlp* m, long long first, int count, float* grad, float lr, int step) {
+    const int rows = (int)std::min<long long>(4LL * m->nsm, ((long long)count + TRAIN_TS - 1) / TRAIN_TS);
+    k_train_grad<<<rows, 256, 0, m->st>>>(m->P, m->x, m->y, m->ok, first, count, 1.f / count, m->part);
+    k_train_update<<<(TRAIN_ROW + 31) / 32, 256, 0, m->st>>>(m->part, rows, m->P, grad, m->M1, m->M2, m->loss, lr,
+                                                             0.9f, 0.999f, 1e-8f, step);
 }
 
 // CTAs of a tcgen05 kernel: the resident ones only (each allocates TMEM once
@@ -646,7 +662,8 @@ int claw2_mlp_create(int device, unsigned long long seed, claw2_mlp** out) {
     DeviceGuard g(device);
     bool ok = cudaMalloc(&m->P, MLP_NPARAM * 4) == cudaSuccess && cudaMalloc(&m->G, MLP_NPARAM * 4) == cudaSuccess &&
               cudaMalloc(&m->M1, MLP_NPARAM * 4) == cudaSuccess && cudaMalloc(&m->M2, MLP_NPARAM * 4) == cudaSuccess &&
-              cudaMalloc(&m->loss, 4) == cudaSuccess && cudaMalloc(&m->packed, sizeof(MlpPacked)) == cudaSuccess &&
+              cudaMalloc(&m->loss, 4) == cudaSuccess &&
+              cudaMalloc(&m->part, sizeof(float) * TRAIN_ROW * train_cap(device)) == cudaSuccess && cudaMalloc(&m->packed, sizeof(MlpPacked)) == cudaSuccess &&
               cudaMalloc(&m->tc, sizeof(MlpTcImage)) == cudaSuccess && cudaMalloc(&m->status, 4) == cudaSuccess &&
               cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) == cudaSuccess;
     if (!ok) {
@@ -673,7 +690,6 @@ int claw2_mlp_create(int device, unsigned long long seed, claw2_mlp** out) {
     fill(OFF_W2, MLP_H, MLP_H);
     fill(OFF_W3, 1, MLP_H);
     cudaMemcpy(m->P, h.data(), MLP_NPARAM * 4, cudaMemcpyHostToDevice);
-    cudaMemset(m->G, 0, MLP_NPARAM * 4);
     cudaMemset(m->M1, 0, MLP_NPARAM * 4);
     cudaMemset(m->M2, 0, MLP_NPARAM * 4);
     int rc = mlp_repack(m);
@@ -691,6 +707,7 @@ int claw2_mlp_destroy(claw2_mlp* m) {
         DeviceGuard g(m->device);
         if (m->st) cudaStreamSynchronize(m->st);
         cudaFree(m->P); cudaFree(m->G); cudaFree(m->M1); cudaFree(m->M2); cudaFree(m->loss);
+        cudaFree(m->part);
         cudaFree(m->packed); cudaFree(m->tc); cudaFree(m->status); cudaFree(m->x); cudaFree(m->y); cudaFree(m->ok);
         if (m->st) cudaStreamDestroy(m->st);
     }
@@ -756,15 +773,12 @@ int claw2_mlp_gradient(claw2_mlp* m, long long first, int count, float* grad, fl
     if (!m || !grad || first < 0 || count < 1 || first + count > m->nsamples)
         return fail(CLAW2_EINVAL, "bad sample range");
     DeviceGuard g(m->device);
-    CUDA_TRY(cudaMemsetAsync(m->G, 0, MLP_NPARAM * 4, m->st));
     CUDA_TRY(cudaMemsetAsync(m->loss, 0, 4, m->st));
-    k_train_grad<<<(count + 255) / 256, 256, 0, m->st>>>(m->P, m->x, m->y, m->ok, first, count, 1.f / count, m->G,
-                                                         m->loss);
+    mlp_batch_launch(m, first, count, m->G, 0.f, 0);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(grad, m->G, MLP_NPARAM * 4, cudaMemcpyDeviceToHost, m->st));
     if (loss) CUDA_TRY(cudaMemcpyAsync(loss, m->loss, 4, cudaMemcpyDeviceToHost, m->st));
     CUDA_TRY(cudaStreamSynchronize(m->st));
-    CUDA_TRY(cudaMemset(m->G, 0, MLP_NPARAM * 4));
     return CLAW2_OK;
 }
 
@@ -776,13 +790,10 @@ int claw2_mlp_train(claw2_mlp* m, int epochs, int batch, float lr, float* last_l
     for (int e = 0; e < epochs; ++e) {
         CUDA_TRY(cudaMemsetAsync(m->loss, 0, 4, m->st));
         for (long long b = 0; b < nb; ++b) {
-            k_train_grad<<<(batch + 255) / 256, 256, 0, m->st>>>(m->P, m->x, m->y, m->ok, b * batch, batch,
-                                                                 1.f / batch, m->G, m->loss);
             ++m->adam_step;
             // step size decays linearly to a tenth over the run
             const float frac = (float)(e * nb + b) / (float)(epochs * nb);
-            k_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(m->P, m->G, m->M1, m->M2, lr * (1.f - 0.9f * frac),
-                                                                0.9f, 0.999f, 1e-8f, m->adam_step);
+            mlp_batch_launch(m, b * batch, batch, nullptr, lr * (1.f - 0.9f * frac), m->adam_step);
         }
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(&l, m->loss, 4, cudaMemcpyDeviceToHost, m->st));

@@ -350,8 +350,8 @@ struct SplitF {
     }
 };
 
-void launch_bc(double* q, const Layout& L, int meqn, const int* bcl, const int* bcu,
-               unsigned long long* cfl_bits, cudaStream_t st, int negate = 1, int part = 0) {
+BCArgs bc_args(double* q, const Layout& L, int meqn, const int* bcl, const int* bcu, unsigned long long* cfl_bits,
+               int negate, int part) {
     BCArgs b;
     b.negate = negate;
     b.part = part;
@@ -361,8 +361,14 @@ void launch_bc(double* q, const Layout& L, int meqn, const int* bcl, const int* 
     b.bcl[0] = bcl[0]; b.bcl[1] = bcl[1];
     b.bcu[0] = bcu[0]; b.bcu[1] = bcu[1];
     b.cfl_bits = cfl_bits;
-    const int n = 4 * (L.mx + 4) + 4 * L.my;
-    k_bc_fill<<<(n + 255) / 256, 256, 0, st>>>(b);
+    return b;
+}
+int bc_blocks(const Layout& L) { return (4 * (L.mx + 4) + 4 * L.my + 255) / 256; }  // of 256 threads
+
+void launch_bc(double* q, const Layout& L, int meqn, const int* bcl, const int* bcu,
+               unsigned long long* cfl_bits, cudaStream_t st, int negate = 1, int part = 0) {
+    const BCArgs b = bc_args(q, L, meqn, bcl, bcu, cfl_bits, negate, part);
+    k_bc_fill<<<bc_blocks(L), 256, 0, st>>>(b);
 }
 
 int check_method(int rp, int order, int trans, const int* mthlim, int mwaves, int fwave) {
@@ -639,15 +645,15 @@ int mlp_tc_grid(const claw2_mlp* m, K kernel, int* per_sm, long long tiles) {
 }
 
 void mlp_guess_launch(claw2_mlp* m, const double* q, const Layout& L, double gamma, double* guess, int* status,
-                      cudaStream_t st) {
+                      cudaStream_t st, const EvolveDev* evo = nullptr, const double* q2 = nullptr) {
     if (m->engine == CLAW2_MLP_TCGEN05) {
         const long long tiles = (long long)((L.mx + 4 + 31) / 32) * ((L.my + 4 + 3) / 4);
         const int grid = mlp_tc_grid(m, k_mlp_guess_tc, &m->guess_per_sm, tiles);
-        k_mlp_guess_tc<<<grid, 128, 0, st>>>(m->tc, q, L, gamma, guess, status);
+        k_mlp_guess_tc<<<grid, 128, 0, st>>>(m->tc, q, L, gamma, guess, status, evo, q2);
         return;
     }
     dim3 grid((L.mx + 4 + 31) / 32, (L.my + 4 + 3) / 4);
-    k_mlp_guess<<<grid, 128, 0, st>>>(m->packed, q, L, gamma, guess);
+    k_mlp_guess<<<grid, 128, 0, st>>>(m->packed, q, L, gamma, guess, evo, q2);
 }
 
 }  // namespace
@@ -843,6 +849,13 @@ int claw2_mlp_set_engine(claw2_mlp* m, int engine) {
 // Device-resident patch
 // ===========================================================================
 struct claw2_mlp;
+// The device time loop's memory.  Attempt k reads record k & 1 and commits its
+// Courant number to word k & 1; the kernel that ends it writes the other record
+// and clears the other word, so no block of it reads what another writes.
+struct EvolveBlock {
+    EvolveDev rec[2];
+    unsigned long long cfl[2];
+};
 struct claw2_patch {
     claw2_desc d;
     Layout L;
@@ -868,8 +881,8 @@ struct claw2_patch {
     double exact_guess_err = 0.0;             // mode 1: relative error put on the converged p*
     int split_part = 0;                       // 1 after claw2_patch_step_part(.., 1): part 2 must follow
     claw2_mlp* mlp = nullptr;
-    // claw2_patch_evolve's captured attempts, one graph per starting buffer
-    // parity, reused while nothing they captured changed: graph_gen counts
+    // claw2_patch_evolve's captured attempts, one graph per parity of the first
+    // attempt (its record), reused while nothing they captured changed: graph_gen counts
     // changes of the patch's parameters, network and tile schedule arrays
     cudaGraphExec_t evo_exec[2] = {nullptr, nullptr};
     unsigned long long evo_stamp[2] = {0, 0};
@@ -895,7 +908,7 @@ struct claw2_patch {
     double* out_host = nullptr;
     cudaEvent_t out_ev = nullptr;
     // claw2_patch_evolve: the time loop's state on the device and a pinned copy
-    EvolveDev* evo = nullptr;
+    EvolveBlock* evo = nullptr;
     EvolveDev* h_evo = nullptr;
     std::thread* writer = nullptr;
     int writer_rc = 0;
@@ -1480,73 +1493,94 @@ __host__ __device__ inline void evolve_get_dt(EvolveDev& e) {
     e.dtdy = e.dt / e.dy;
 }
 
-// After one step of the loop (one thread): the reference's accept/reject
-// (solver.py:554-666): accept when cfl <= cfl_max (t += dt, or t = tstart +
-// (n + 1) dt with a fixed dt); a rejected step keeps t and is restored by
-// k_evolve_restore (a fixed dt ends the loop with cfl_error); the loop is
+// The end of an attempt: the reference's accept/reject (solver.py:554-666).
+// Accept when cfl <= cfl_max (t += dt, or t = tstart + (n + 1) dt with a fixed
+// dt) and make the step's buffer the current one; a rejected step keeps t and
+// the current buffer (a fixed dt ends the loop with cfl_error); the loop is
 // done when t >= tend, after max_steps attempts, or when the step produced a
-// non-finite value (fault, the step restored); otherwise the next dt.
-static __global__ void k_evolve_finalize(EvolveDev* e, const unsigned long long* cfl_bits, const int* status) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || e->done) return;
-    const double cfl = __longlong_as_double((long long)*cfl_bits);
-    const int n = e->attempts;
-    e->attempts = n + 1;
-    e->cfl = cfl;
-    const int st = *status & 3;
+// non-finite value (fault, the step dropped); otherwise the next dt.  Returns
+// true when the next attempt starts from a new buffer, whose ghost cells are
+// still to be filled.
+__device__ __forceinline__ bool evolve_finish(EvolveDev& e, double cfl, int status) {
+    const int n = e.attempts;
+    e.attempts = n + 1;
+    e.cfl = cfl;
+    const int st = status & 3;
     if (st) {
-        e->fault = st;
-        e->reject = 1;
-        e->done = 1;
-        return;
+        e.fault = st;
+        e.done = 1;
+        return false;
     }
-    if (!(cfl > e->cfl_max)) {
-        e->cflmax = (e->cflmax > cfl) ? e->cflmax : cfl;  // max(cfl, cflmax)
-        e->t = e->dt_variable ? __dadd_rn(e->t, e->dt) : __dadd_rn(e->tstart, __dmul_rn((double)(n + 1), e->dt));
-        e->num_steps += 1;
-        e->reject = 0;
-    } else {
-        e->reject = 1;
-        if (!e->dt_variable) {
-            e->cflmax = (e->cflmax > cfl) ? e->cflmax : cfl;
-            e->cfl_error = 1;
-            e->done = 1;
-            return;
+    const bool accept = !(cfl > e.cfl_max);
+    if (accept) {
+        e.cflmax = (e.cflmax > cfl) ? e.cflmax : cfl;  // max(cfl, cflmax)
+        e.t = e.dt_variable ? __dadd_rn(e.t, e.dt) : __dadd_rn(e.tstart, __dmul_rn((double)(n + 1), e.dt));
+        e.num_steps += 1;
+        e.cur ^= 1;
+    } else if (!e.dt_variable) {
+        e.cflmax = (e.cflmax > cfl) ? e.cflmax : cfl;
+        e.cfl_error = 1;
+        e.done = 1;
+        return false;
+    }
+    if (e.t >= e.tend || e.attempts >= e.max_steps) {
+        e.done = 1;
+        return false;
+    }
+    evolve_get_dt(e);
+    return accept;
+}
+
+// One launch ends an attempt and prepares the next: every block works out the
+// decision for itself from the attempt's record and Courant number (block 0
+// writes it down, into the other record), then fills its share of the ghost
+// cells of the new current buffer.  A rejected attempt costs nothing more:
+// its record keeps naming the old buffer, whose ghost cells are still valid.
+// It stands for three launches (one-thread finalize, copy back on reject,
+// ghost fill), 10.7 us of the 21 us an attempt took at 200^2; latency bound.
+static __global__ void __launch_bounds__(256) k_evolve_next(const EvolveDev* in, EvolveDev* out,
+                                                            const unsigned long long* cfl, unsigned long long* next_cfl,
+                                                            const int* status, double* q0, double* q1, const BCArgs b) {
+    __shared__ int fill;
+    if (threadIdx.x == 0) {
+        EvolveDev e = *in;
+        const double c = __longlong_as_double((long long)*cfl);
+        const int st = *status;
+        int f = -1;
+        const bool was_done = e.done;
+        if (!was_done && evolve_finish(e, c, st)) f = e.cur;
+        if (blockIdx.x == 0) {
+            *out = e;
+            if (!was_done) *next_cfl = 0ull;  // (the last attempt's word stays for claw2_patch_cfl)
         }
+        fill = f;
     }
-    if (e->t >= e->tend || e->attempts >= e->max_steps) {
-        e->done = 1;
-        return;
-    }
-    evolve_get_dt(*e);
+    __syncthreads();
+    if (fill < 0) return;
+    bc_fill_cell(b, fill ? q1 : q0, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// A rejected step: the state it started from continues in the other buffer.
-static __global__ void k_evolve_restore(const EvolveDev* e, const double* __restrict__ from, double* __restrict__ to,
-                                        long long n) {
-    if (!e->reject) return;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x)
-        to[k] = from[k];
-}
-
-// One attempt of the loop from buffer c: ghost fill, step into buffer 1-c
-// with the loop's dt, finalize, restore on reject.
+// One attempt of the loop with the record of parity c: step from the record's
+// current buffer into the other with its dt, then the decision, the next dt
+// and the next state's ghost cells.
 int evolve_enqueue_attempt(claw2_patch* p, int c) {
-    double* qc = p->q[c];
-    launch_bc(qc, p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, p->cfl, p->st);
+    EvolveDev* rec = &p->evo->rec[c];
     StepArgs a = patch_args(p, 0.0);
-    a.qold = p->q[c];
-    a.qnew = p->q[c ^ 1];
-    a.evo = p->evo;
+    a.qold = p->q[0];
+    a.qnew = p->q[1];
+    a.qold2 = p->q[1];
+    a.qnew2 = p->q[0];
+    a.evo = rec;
+    a.cfl_bits = &p->evo->cfl[c];
     if (p->d.riemann == CLAW2_RP_EULER_EXACT && p->mlp && !p->d.dimensional_split) {
-        mlp_guess_launch(p->mlp, qc, p->L, p->rp.c[0], p->guess, p->status, p->st);
+        mlp_guess_launch(p->mlp, p->q[0], p->L, p->rp.c[0], p->guess, p->status, p->st, rec, p->q[1]);
         a.guess = p->guess;
     }
     int lpt_n = 0;
     if (p->d.dimensional_split) {
         StepArgs ax = a, ay = a;
-        ax.qnew = p->tmp;
-        ay.qold = p->tmp;
+        ax.qnew = ax.qnew2 = p->tmp;
+        ay.qold = ay.qold2 = p->tmp;
         dispatch<SplitF>(p->d.riemann, ax, ay, p->st, 3);
     } else {
         int ns, H, nb;
@@ -1558,15 +1592,12 @@ int evolve_enqueue_attempt(claw2_patch* p, int c) {
             a.tile_order = p->tile_order;
             a.tile_cost = p->tile_cost;
         }
-        dispatch<UnsplitF>(p->d.riemann, a, p->st, p->has_tmap ? &p->tmap[c] : nullptr);
+        dispatch<UnsplitF>(p->d.riemann, a, p->st, nullptr);
     }
     if (lpt_n > 0 && (p->tile_steps++ % LPT_EVERY) == 0) launch_lpt(p->tile_cost, p->tile_order, lpt_n, p->st);
-    k_evolve_finalize<<<1, 32, 0, p->st>>>(p->evo, p->cfl, p->status);
-    const long long n = (long long)p->d.num_eqn * p->L.plane;
-    // grid-stride copy on a few blocks per SM: accepted attempts (almost all)
-    // leave it at once, so its launch stays short
-    const int rb = (int)std::max<long long>(1, std::min<long long>(grid_blocks(n), 4LL * p->nsm));
-    k_evolve_restore<<<rb, 256, 0, p->st>>>(p->evo, p->q[c], p->q[c ^ 1], n);
+    const BCArgs b = bc_args(nullptr, p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, nullptr, 1, 0);
+    k_evolve_next<<<bc_blocks(p->L), 256, 0, p->st>>>(rec, &p->evo->rec[c ^ 1], &p->evo->cfl[c], &p->evo->cfl[c ^ 1],
+                                                     p->status, p->q[0], p->q[1], b);
     CUDA_TRY(cudaGetLastError());
     return CLAW2_OK;
 }
@@ -1653,7 +1684,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     if (s->max_steps == 0) return CLAW2_OK;
     DeviceGuard g(p->device);
     if (!p->evo) {
-        if (cudaMalloc(&p->evo, sizeof(EvolveDev)) != cudaSuccess ||
+        if (cudaMalloc(&p->evo, sizeof(EvolveBlock)) != cudaSuccess ||
             cudaMallocHost(&p->h_evo, sizeof(EvolveDev)) != cudaSuccess) {
             cudaGetLastError();
             cudaFree(p->evo);
@@ -1679,27 +1710,43 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     e.dt_variable = s->dt_variable ? 1 : 0;
     e.dt_old_set = s->dt_old_set ? 1 : 0;
     e.max_steps = s->max_steps;
+    e.cur = p->cur;
+    // a dt that follows from a Courant number says how many attempts are left;
+    // a first dt is the caller's guess
+    const bool dt_known = e.dt_variable ? e.dt_old_set && e.cfl > 0.0 : true;
     evolve_get_dt(e);  // the first attempt's dt
-    CUDA_TRY(cudaMemcpyAsync(p->evo, p->h_evo, sizeof(EvolveDev), cudaMemcpyHostToDevice, p->st));
+    CUDA_TRY(cudaMemcpyAsync(&p->evo->rec[0], p->h_evo, sizeof(EvolveDev), cudaMemcpyHostToDevice, p->st));
     CUDA_TRY(cudaMemsetAsync(p->status, 0, sizeof(int), p->st));
-    const int cur0 = p->cur;
+    launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
     long long issued = 0;
-    int chunk = 4;
+    // Attempts are issued in chunks, and the host waits for the record after
+    // each.  A chunk is the number of attempts that the current dt leaves to
+    // tend plus one (an attempt issued too many costs its launches, which do
+    // nothing; one too few costs the host's round trip), at most 64; 4 while dt
+    // is still the caller's guess.
+    auto chunk_of = [](const EvolveDev& r, bool known) {
+        const double left = r.dt > 0.0 ? std::ceil((r.tend - r.t) / r.dt) + 1.0 : 64.0;
+        const double most = std::min(known ? 64.0 : 4.0, (double)(r.max_steps - r.attempts));
+        return (int)std::max(1.0, std::min(left, most));
+    };
+    int chunk = chunk_of(e, dt_known);
     // After the first chunk (issued directly: it also sets up launch attributes
     // and schedule buffers) four attempts are captured as one CUDA graph and
-    // replayed: four attempts return to the same buffer parity, so the same
-    // graph serves every later chunk, and the host no longer pays one launch
-    // per kernel.  The graph is kept for the next call from the same parity
-    // while nothing it captured has changed.  Any capture failure falls back
-    // to direct launches.
+    // replayed: four attempts return to the same record, so the same graph
+    // serves every later chunk, and the host no longer pays one launch per
+    // kernel.  The graph is kept for the next call from the same parity while
+    // nothing it captured has changed.  Any capture failure falls back to
+    // direct launches, which also make up a chunk's last one to three attempts.
     cudaGraphExec_t exec = nullptr;
     constexpr int GRAPH_ATTEMPTS = 4;
     bool try_graph = true;
+    int exec_parity = -1;
     int rc = CLAW2_OK;
     for (;;) {
-        if (issued > 0 && try_graph && !exec) {
-            try_graph = false;
-            const int c = (int)((cur0 + issued) & 1);
+        if (issued > 0 && chunk >= GRAPH_ATTEMPTS && (issued & 1) != exec_parity) exec = nullptr;
+        if (issued > 0 && chunk >= GRAPH_ATTEMPTS && try_graph && !exec) {
+            const int c = (int)(issued & 1);
+            exec_parity = c;
             const unsigned long long stamp =
                 ((unsigned long long)p->graph_gen << 32) | (unsigned long long)g_tune_gen.load();
             if (p->evo_exec[c] && p->evo_stamp[c] == stamp) {
@@ -1715,6 +1762,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
                     exec = nullptr;
                 }
                 if (graph) cudaGraphDestroy(graph);
+                try_graph = exec != nullptr;
                 if (exec) {
                     if (p->evo_exec[c]) cudaGraphExecDestroy(p->evo_exec[c]);
                     p->evo_exec[c] = exec;
@@ -1722,20 +1770,20 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
                 }
             } else {
                 cudaGetLastError();
+                try_graph = false;
             }
         }
-        if (exec) {
-            for (int j = 0; j < chunk; j += GRAPH_ATTEMPTS, issued += GRAPH_ATTEMPTS)
+        if (exec && exec_parity == (issued & 1)) {
+            for (; chunk >= GRAPH_ATTEMPTS; chunk -= GRAPH_ATTEMPTS, issued += GRAPH_ATTEMPTS)
                 if (cudaGraphLaunch(exec, p->st) != cudaSuccess) {
                     rc = fail(CLAW2_ECUDA, "graph launch of the time loop failed");
                     break;
                 }
-        } else {
-            for (int j = 0; j < chunk && rc == CLAW2_OK; ++j, ++issued)
-                rc = evolve_enqueue_attempt(p, (int)((cur0 + issued) & 1));
         }
+        for (; chunk > 0 && rc == CLAW2_OK; --chunk, ++issued) rc = evolve_enqueue_attempt(p, (int)(issued & 1));
         if (rc == CLAW2_OK) {
-            if (cudaMemcpyAsync(p->h_evo, p->evo, sizeof(EvolveDev), cudaMemcpyDeviceToHost, p->st) != cudaSuccess ||
+            if (cudaMemcpyAsync(p->h_evo, &p->evo->rec[issued & 1], sizeof(EvolveDev), cudaMemcpyDeviceToHost,
+                                p->st) != cudaSuccess ||
                 cudaStreamSynchronize(p->st) != cudaSuccess)
                 rc = fail(CLAW2_ECUDA, "reading the time loop's state failed");
         }
@@ -1744,10 +1792,13 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
             rc = fail(CLAW2_ECUDA, "the device time loop did not finish");
             break;
         }
-        chunk = std::min(chunk * 2, 64);
+        chunk = chunk_of(e, true);
     }
     if (rc != CLAW2_OK) return rc;
-    p->cur = (cur0 + e.attempts) & 1;
+    p->cur = e.cur;
+    // claw2_patch_cfl after the loop: the last attempt's Courant number
+    cudaMemcpyAsync(p->cfl, &p->evo->cfl[(e.attempts - 1) & 1], sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
+                    p->st);
     s->t = e.t;
     s->dt = e.dt;
     s->cfl = e.cfl;

@@ -458,8 +458,12 @@ static __global__ void k_mlp_eval(const MlpPacked* __restrict__ Mg, const float*
 // x-interface (cp-1 | cp) on row R and the y-interface (R-1 | R) on column cp.
 // guess planes: [0] x-interfaces, [1] y-interfaces, q's layout.
 static __global__ void __launch_bounds__(128) k_mlp_guess(const MlpPacked* __restrict__ Mg,
-                                                          const double* __restrict__ q, Layout L, double gamma,
-                                                          double* guess) {
+                                                          const double* q, Layout L, double gamma, double* guess,
+                                                          const EvolveDev* evo, const double* q2) {
+    if (evo) {  // the device time loop's record: nothing to do, or the other buffer
+        if (evo->done) return;
+        if (evo->cur) q = q2;
+    }
     __shared__ MlpPacked M;
     __shared__ float rows[4][64][8];
     __shared__ float res[4][64];
@@ -817,8 +821,12 @@ __device__ __forceinline__ void features_f32(float g, const double (&a)[5], cons
 // x-interface (cp-1 | cp) on row R (tile 0, row t) and the y-interface
 // (R-1 | R) on column cp (tile 1, row t).  CTAs loop over the site tiles.
 static __global__ void __launch_bounds__(128, 5) k_mlp_guess_tc(const MlpTcImage* __restrict__ Mg,
-                                                             const double* __restrict__ q, Layout L, double gamma,
-                                                             double* guess, int* status) {
+                                                             const double* q, Layout L, double gamma, double* guess,
+                                                             int* status, const EvolveDev* evo, const double* q2) {
+    if (evo) {  // the device time loop's record: nothing to do, or the other buffer
+        if (evo->done) return;
+        if (evo->cur) q = q2;
+    }
     __shared__ MlpTcSmem S;
     __shared__ double sprim[4][5][32];  // each warp's cells (rho, u, v, p, c): the row above's lower neighbours
     mlp_tc_setup(S, Mg);

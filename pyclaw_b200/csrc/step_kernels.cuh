@@ -32,11 +32,13 @@
 namespace claw2 {
 
 // Device-resident time loop (claw2_patch_evolve): the loop's state lives in
-// device memory; each step reads its dt/dx, dt/dy from it and does nothing
-// once the loop is done.  Field meanings as in claw2_evolve_state.
+// device memory; each step reads its dt/dx, dt/dy and which buffer holds the
+// current state from it and does nothing once the loop is done.  Field
+// meanings as in claw2_evolve_state.
 struct EvolveDev {
     double t, tstart, tend, dt, dtdx, dtdy, cfl, cfl_desired, cfl_max, dt_max, dtmin, dtmax, cflmax, dx, dy;
-    int dt_variable, dt_old_set, max_steps, attempts, num_steps, cfl_error, done, reject, fault;
+    int dt_variable, dt_old_set, max_steps, attempts, num_steps, cfl_error, done, fault;
+    int cur;  // the buffer of the current state
 };
 
 struct StepArgs {
@@ -63,14 +65,28 @@ struct StepArgs {
     int tile_offset = 0, tile_jump_at = 1 << 30, tile_jump = 0, tile_count = 0;
     // aux planes (same layout as q) for solvers with aux data, else nullptr
     const double* __restrict__ aux = nullptr;
-    // device-resident time loop: dt from here, no work once it is done (else nullptr)
+    // device-resident time loop: dt and the current buffer from here, no work
+    // once it is done (else nullptr); with buffer 1 current the step reads
+    // qold2 and writes qnew2 instead
     const EvolveDev* evo = nullptr;
+    const double* qold2 = nullptr;
+    double* qnew2 = nullptr;
     // capacity function kappa (one plane, same layout), else nullptr: every
     // increment of a cell is divided by its kappa, a transverse increment also
     // by the kappa of the cell its fluctuation entered (step2.f90:132-160,
     // flux2.f90:104-119,134-203 with dtdx1d = dtdx / kappa)
     const double* __restrict__ capa = nullptr;
 };
+
+// The buffers a step reads and writes (EVO: the loop's record names them).
+template <bool EVO>
+__device__ __forceinline__ const double* step_in(const StepArgs& a) {
+    return (EVO && a.evo->cur) ? a.qold2 : a.qold;
+}
+template <bool EVO>
+__device__ __forceinline__ double* step_out(const StepArgs& a) {
+    return (EVO && a.evo->cur) ? a.qnew2 : a.qnew;
+}
 
 // The tile a CTA of a step launch runs (see StepArgs::tile_order, tile_offset).
 __device__ __forceinline__ int tile_index(const StepArgs& a) {
@@ -362,8 +378,8 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
     const int order = (SPEC == SPEC_MC2) ? 2 : a.meth.order;
     const int trans = (SPEC == SPEC_MC2) ? 2 : a.meth.transverse;
     const bool tc = (order > 1) && (trans == 2);
-    const double* qo = a.qold + cpl;
-    double* qn = a.qnew + cpl;
+    const double* qo = step_in<EVO>(a) + cpl;
+    double* qn = step_out<EVO>(a) + cpl;
 
     // aux data: loaded with q a row ahead (MA planes); solvers whose transverse
     // solve needs the cells above and below (TAUX) run the x-interface's
@@ -945,8 +961,8 @@ __global__ void __launch_bounds__(NT) k_split_x(const StepArgs a) {
     const int tr = (t < NT - 1) ? t + 1 : NT - 1;
     const double dtdx = EVO ? a.evo->dtdx : a.dtdx;  // (compile-time choice, as in unsplit_tile)
     const RPParams& P = a.rp;
-    const double* qo = a.qold + cpl;
-    double* qn = a.qnew + cpl;
+    const double* qo = step_in<EVO>(a) + cpl;
+    double* qn = step_out<EVO>(a) + cpl;
     double cfl = 0.0;
     // zero-jump shortcut (q-wave solvers without aux data), as in unsplit_tile
     constexpr bool ZS = SkipTraits<RP>::OK && AuxTraits<RP>::MAUX == 0;
@@ -1049,8 +1065,8 @@ __global__ void __launch_bounds__(NT) k_split_y(const StepArgs a) {
     const int R0 = rb, R1 = rb + Hb + 3;
     const double dtdy = EVO ? a.evo->dtdy : a.dtdy;
     const RPParams& P = a.rp;
-    const double* qo = a.qold + cpl;
-    double* qn = a.qnew + cpl;
+    const double* qo = step_in<EVO>(a) + cpl;
+    double* qn = step_out<EVO>(a) + cpl;
 
     // zero-jump shortcut (q-wave solvers without aux data), as in unsplit_tile
     constexpr bool ZS = SkipTraits<RP>::OK && AuxTraits<RP>::MAUX == 0;
@@ -1204,12 +1220,12 @@ __device__ __forceinline__ int bc_src(int c, int n, int lo, int up, bool& flip) 
     return c;
 }
 
-static __global__ void k_bc_fill(const BCArgs a) {
+// Ghost cell k of the buffer q (k counts the 4 ghost rows, then the ghost
+// columns of the interior rows; larger k do nothing).
+__device__ __forceinline__ void bc_fill_cell(const BCArgs& a, double* q, int k) {
     const int mx = a.L.mx, my = a.L.my;
     const int nrow = 4 * (mx + 4);   // cells of the 4 ghost rows
     const int ncol = 4 * my;         // ghost-column cells of interior rows
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0 && a.cfl_bits && a.part != 2) *a.cfl_bits = 0ull;
     if (k >= nrow + ncol) return;
     int c, r;
     if (k < nrow) {
@@ -1239,7 +1255,7 @@ static __global__ void k_bc_fill(const BCArgs a) {
         double v[G];
 #pragma unroll
         for (int k = 0; k < G; ++k)
-            if (m0 + k < a.meqn) v[k] = a.q[(m0 + k) * a.L.plane + src];
+            if (m0 + k < a.meqn) v[k] = q[(m0 + k) * a.L.plane + src];
 #pragma unroll
         for (int k = 0; k < G; ++k) {
             const int m = m0 + k;
@@ -1247,9 +1263,15 @@ static __global__ void k_bc_fill(const BCArgs a) {
             double x = v[k];
             if (a.negate && fx && m == 1) x = -x;
             if (a.negate && fy && m == 2) x = -x;
-            a.q[m * a.L.plane + dst] = x;
+            q[m * a.L.plane + dst] = x;
         }
     }
+}
+
+static __global__ void k_bc_fill(const BCArgs a) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == 0 && a.cfl_bits && a.part != 2) *a.cfl_bits = 0ull;
+    bc_fill_cell(a, a.q, k);
 }
 
 // ---------------------------------------------------------------------------

@@ -20,6 +20,7 @@
 
 #include "batch.cuh"
 #include "mlp.cuh"
+#include "small_grid.cuh"
 #include "step_kernels.cuh"
 
 #include <vector>
@@ -855,6 +856,7 @@ struct claw2_mlp;
 struct EvolveBlock {
     EvolveDev rec[2];
     unsigned long long cfl[2];
+    SmallCtl ctl;  // of the small-grid loop
 };
 struct claw2_patch {
     claw2_desc d;
@@ -1472,65 +1474,6 @@ int patch_enqueue_step(claw2_patch* p, double dt, int part = 0) {
 // ---------------------------------------------------------------------------
 // Device-resident time loop (claw2_patch_evolve)
 // ---------------------------------------------------------------------------
-// get_dt of the reference's loop (src/pyclaw/solver.py:524-552) on the loop
-// state, with Python's min/max tie rules (same values), then dt/dx, dt/dy.
-__host__ __device__ inline void evolve_get_dt(EvolveDev& e) {
-    if (e.dt_variable && e.dt_old_set) {
-        if (e.cfl > 0.0) {
-            const double x = e.dt * e.cfl_desired / e.cfl;
-            e.dt = (x < e.dt_max) ? x : e.dt_max;             // min(dt_max, x)
-            e.dtmin = (e.dtmin < e.dt) ? e.dtmin : e.dt;      // min(dt, dtmin)
-            e.dtmax = (e.dtmax > e.dt) ? e.dtmax : e.dt;      // max(dt, dtmax)
-        } else {
-            e.dt = e.dt_max;
-        }
-    } else {
-        e.dt_old_set = 1;
-    }
-    if (e.t + e.dt > e.tend && e.tstart < e.tend) e.dt = e.tend - e.t;
-    if (e.tend - e.t - e.dt < 1.e-14 * e.t) e.dt = e.tend - e.t;
-    e.dtdx = e.dt / e.dx;
-    e.dtdy = e.dt / e.dy;
-}
-
-// The end of an attempt: the reference's accept/reject (solver.py:554-666).
-// Accept when cfl <= cfl_max (t += dt, or t = tstart + (n + 1) dt with a fixed
-// dt) and make the step's buffer the current one; a rejected step keeps t and
-// the current buffer (a fixed dt ends the loop with cfl_error); the loop is
-// done when t >= tend, after max_steps attempts, or when the step produced a
-// non-finite value (fault, the step dropped); otherwise the next dt.  Returns
-// true when the next attempt starts from a new buffer, whose ghost cells are
-// still to be filled.
-__device__ __forceinline__ bool evolve_finish(EvolveDev& e, double cfl, int status) {
-    const int n = e.attempts;
-    e.attempts = n + 1;
-    e.cfl = cfl;
-    const int st = status & 3;
-    if (st) {
-        e.fault = st;
-        e.done = 1;
-        return false;
-    }
-    const bool accept = !(cfl > e.cfl_max);
-    if (accept) {
-        e.cflmax = (e.cflmax > cfl) ? e.cflmax : cfl;  // max(cfl, cflmax)
-        e.t = e.dt_variable ? __dadd_rn(e.t, e.dt) : __dadd_rn(e.tstart, __dmul_rn((double)(n + 1), e.dt));
-        e.num_steps += 1;
-        e.cur ^= 1;
-    } else if (!e.dt_variable) {
-        e.cflmax = (e.cflmax > cfl) ? e.cflmax : cfl;
-        e.cfl_error = 1;
-        e.done = 1;
-        return false;
-    }
-    if (e.t >= e.tend || e.attempts >= e.max_steps) {
-        e.done = 1;
-        return false;
-    }
-    evolve_get_dt(e);
-    return accept;
-}
-
 // One launch ends an attempt and prepares the next: every block works out the
 // decision for itself from the attempt's record and Courant number (block 0
 // writes it down, into the other record), then fills its share of the ghost
@@ -1551,13 +1494,83 @@ static __global__ void __launch_bounds__(256) k_evolve_next(const EvolveDev* in,
         if (!was_done && evolve_finish(e, c, st)) f = e.cur;
         if (blockIdx.x == 0) {
             *out = e;
-            if (!was_done) *next_cfl = 0ull;  // (the last attempt's word stays for claw2_patch_cfl)
+            *next_cfl = 0ull;
         }
         fill = f;
     }
     __syncthreads();
     if (fill < 0) return;
     bc_fill_cell(b, fill ? q1 : q0, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// The small-grid loop (small_grid.cuh): tile height, and a launch of up to
+// `budget` attempts on rec[0].
+template <class RP>
+struct SmallF {
+    static constexpr int NY = sizeof(SmallSmem<RP, 16>) <= 220 * 1024 ? 16 : 8;
+    static_assert(sizeof(SmallSmem<RP, NY>) <= 220 * 1024, "the tile must fit in shared memory");
+    template <int SPEC, bool SPLIT>
+    static cudaError_t go(const StepArgs& a, const BCArgs& b, EvolveBlock* e, int budget, int grid, cudaStream_t st) {
+        auto kern = k_small_evolve<RP, NY, SPEC, SPLIT>;
+        constexpr int smem = (int)sizeof(SmallSmem<RP, NY>);
+        static unsigned long long attr = 0;
+        smem_attr(kern, smem, attr);
+        StepArgs aa = a;
+        BCArgs bb = b;
+        EvolveDev* rec = &e->rec[0];
+        SmallCtl* ctl = &e->ctl;
+        void* args[] = {&aa, &bb, &rec, &ctl, &budget};
+        return cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(32 * NY), args, smem, st);
+    }
+    static void run(const StepArgs& a, const BCArgs& b, EvolveBlock* e, int budget, bool split, int nsm,
+                    cudaStream_t st, cudaError_t* rc) {
+        if constexpr (!GuessTraits<RP>::USES) {
+            const int tiles = ((a.L.mx + 27) / 28) * ((a.L.my + NY - 5) / (NY - 4));
+            const int grid = std::min(tiles, nsm);
+            if (split) {
+                switch (split_spec(a.meth, RP::MWAVES)) {
+                    case SPEC_MC2: *rc = go<SPEC_MC2, true>(a, b, e, budget, grid, st); break;
+                    case SPEC_MM2: *rc = go<SPEC_MM2, true>(a, b, e, budget, grid, st); break;
+                    default: *rc = go<SPEC_ANY, true>(a, b, e, budget, grid, st); break;
+                }
+            } else if (is_mc2(a.meth, RP::MWAVES)) {
+                *rc = go<SPEC_MC2, false>(a, b, e, budget, grid, st);
+            } else {
+                *rc = go<SPEC_ANY, false>(a, b, e, budget, grid, st);
+            }
+        } else {
+            *rc = cudaErrorNotSupported;
+        }
+    }
+};
+template <class RP>
+struct SmallTilesF {
+    static void run(int mx, int my, int* tiles) {
+        if constexpr (!GuessTraits<RP>::USES)
+            *tiles = ((mx + 27) / 28) * ((my + SmallF<RP>::NY - 5) / (SmallF<RP>::NY - 4));
+        else *tiles = -1;  // (a guess per interface: marching kernels only)
+    }
+};
+
+// Whether the time loop of a patch runs as the small-grid kernel.  Measured per
+// step, marching kernels against it (acoustics / shallow water / Euler, MC):
+// split, 200^2 17.4 -> 8.0 / 20.3 -> 8.9 / 21.6 -> 9.9 us, 800^2 37.6 -> 27 / 51 -> 38 /
+// 78 -> 54 us and 2500^2 273 -> 204 / 317 -> 260 / 572 -> 407 us: always.  Unsplit,
+// 200^2 15.0 -> 8.3 / 18.7 -> 9.7 / 23.3 -> 11 us, 800^2 35 -> 36 / 49 -> 40 / 83 -> 72 us,
+// 1600^2 about 95 -> 126 / 140 -> 131 / 230 -> 233 us: while the tiles are at most a
+// dozen per SM (750^2), since a tile computes its halo rows again and a
+// marching strip does not.
+bool small_grid_fits(const claw2_patch* p) {
+    if (p->d.mcapa > 0) return false;  // the capacity form has no small-grid tile
+    for (int d = 0; d < 2; ++d)
+        if (p->d.bc_lower[d] == CLAW2_BC_NONE || p->d.bc_upper[d] == CLAW2_BC_NONE) return false;
+    int tiles = -1;
+    dispatch<SmallTilesF>(p->d.riemann, p->d.mx, p->d.my, &tiles);
+    if (tiles < 0) return false;
+    if (p->d.dimensional_split) return true;
+    const UnsplitShape sh = g_tune[p->d.riemann & (TUNE_SLOTS - 1)];
+    if (sh.variant != 0 || sh.rows != 0) return false;  // the caller asked for a marching shape
+    return tiles <= 12 * p->nsm;
 }
 
 // One attempt of the loop with the record of parity c: step from the record's
@@ -1717,7 +1730,8 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     evolve_get_dt(e);  // the first attempt's dt
     CUDA_TRY(cudaMemcpyAsync(&p->evo->rec[0], p->h_evo, sizeof(EvolveDev), cudaMemcpyHostToDevice, p->st));
     CUDA_TRY(cudaMemsetAsync(p->status, 0, sizeof(int), p->st));
-    launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
+    bool small = small_grid_fits(p);
+    if (!small) launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
     long long issued = 0;
     // Attempts are issued in chunks, and the host waits for the record after
     // each.  A chunk is the number of attempts that the current dt leaves to
@@ -1743,6 +1757,29 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     int exec_parity = -1;
     int rc = CLAW2_OK;
     for (;;) {
+        if (small) {  // the whole loop in one launch (again after a budget of attempts)
+            constexpr int BUDGET = 1024;
+            cudaError_t er = cudaMemsetAsync(&p->evo->ctl, 0, sizeof(SmallCtl), p->st);
+            if (er == cudaSuccess) {
+                StepArgs a = patch_args(p, 0.0);
+                a.qold = a.qnew2 = p->q[0];
+                a.qnew = p->q[1];
+                a.qold2 = p->q[1];
+                const BCArgs b = bc_args(nullptr, p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, nullptr, 1, 0);
+                dispatch<SmallF>(p->d.riemann, a, b, p->evo, BUDGET, p->d.dimensional_split != 0, p->nsm, p->st, &er);
+            }
+            if (er == cudaSuccess) {
+                issued += 2 * BUDGET;
+                chunk = 0;
+            } else if (issued > 0) {
+                rc = fail(CLAW2_ECUDA, "the small-grid loop could not continue: %s", cudaGetErrorString(er));
+                chunk = 0;
+            } else {  // no cooperative launch to be had: the marching kernels
+                cudaGetLastError();
+                small = false;
+                launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
+            }
+        }
         if (issued > 0 && chunk >= GRAPH_ATTEMPTS && (issued & 1) != exec_parity) exec = nullptr;
         if (issued > 0 && chunk >= GRAPH_ATTEMPTS && try_graph && !exec) {
             const int c = (int)(issued & 1);
@@ -1788,7 +1825,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
                 rc = fail(CLAW2_ECUDA, "reading the time loop's state failed");
         }
         if (rc != CLAW2_OK || e.done) break;
-        if (issued > (long long)s->max_steps + 128) {  // the loop marks itself done after max_steps attempts
+        if (!small && issued > (long long)s->max_steps + 128) {  // the loop marks itself done after max_steps attempts
             rc = fail(CLAW2_ECUDA, "the device time loop did not finish");
             break;
         }
@@ -1797,8 +1834,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     if (rc != CLAW2_OK) return rc;
     p->cur = e.cur;
     // claw2_patch_cfl after the loop: the last attempt's Courant number
-    cudaMemcpyAsync(p->cfl, &p->evo->cfl[(e.attempts - 1) & 1], sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
-                    p->st);
+    cudaMemcpyAsync(p->cfl, &p->evo->rec[issued & 1].cfl, sizeof(double), cudaMemcpyDeviceToDevice, p->st);
     s->t = e.t;
     s->dt = e.dt;
     s->cfl = e.cfl;
@@ -1811,7 +1847,8 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     s->cfl_error = e.cfl_error;
     if (e.fault) {
         cudaMemsetAsync(p->status, 0, sizeof(int), p->st);
-        if (e.fault & 2) return fail(CLAW2_ETIMEOUT, "a TMA row copy did not complete within the kernel's wait bound");
+        if (e.fault & 2)
+            return fail(CLAW2_ETIMEOUT, "a wait of the time loop (a row copy or the CTAs' barrier) gave up");
         return fail(CLAW2_ENONFINITE, "the step produced a non-finite value");
     }
     return CLAW2_OK;

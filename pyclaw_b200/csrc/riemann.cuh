@@ -1039,8 +1039,9 @@ struct RPVcAcoustics {
         const double zr = cR[ZZ], zl = cL[ZZ];
         const double delta1 = cR[0] - cL[0];
         const double delta2 = cR[MU] - cL[MU];
-        f.alpha[0] = (-delta1 + zr * delta2) / (zl + zr);
-        f.alpha[1] = (delta1 + zl * delta2) / (zl + zr);
+        const double iz = rcp_nr(zl + zr);
+        f.alpha[0] = (-delta1 + zr * delta2) * iz;
+        f.alpha[1] = (delta1 + zl * delta2) * iz;
         f.zl = zl; f.zr = zr; f.cl = cL[CC]; f.cr = cR[CC];
         double w[MWAVES][MEQN], s[MWAVES];
         waves<IXY>(f, p, w);
@@ -1059,10 +1060,37 @@ struct RPVcAcoustics {
                                                     double (&bm)[MEQN], double (&bp)[MEQN]) {
         constexpr int MU = Dir<IXY>::MU, MV = Dir<IXY>::MV;
         const double zm = cm[ZZ], zz = c0[ZZ], zp = cp[ZZ];
-        const double a1 = (-asdq[0] + asdq[MV] * zz) / (zm + zz);
-        const double a2 = (asdq[0] + asdq[MV] * zz) / (zz + zp);
+        const double a1 = (-asdq[0] + asdq[MV] * zz) * rcp_nr(zm + zz);
+        const double a2 = (asdq[0] + asdq[MV] * zz) * rcp_nr(zz + zp);
         bm[0] = cm[CC] * a1 * zm; bm[MU] = 0.0; bm[MV] = -cm[CC] * a1;
         bp[0] = cp[CC] * a2 * zp; bp[MU] = 0.0; bp[MV] = cp[CC] * a2;
+    }
+    // eigenvectors (-zl, 1, 0) and (zr, 1, 0)
+    static constexpr int NLIM = 4;
+    template <int IXY>
+    __device__ __forceinline__ static void lim_rec(const Iface& f, const RPParams&, double (&r)[NLIM]) {
+        r[0] = f.alpha[0]; r[1] = f.alpha[1]; r[2] = f.zl; r[3] = f.zr;
+    }
+    __device__ __forceinline__ static void lim_cross(const double (&x)[NLIM], const double (&y)[NLIM],
+                                                     double (&X)[MWAVES]) {
+        X[0] = 1.0 + x[2] * y[2];
+        X[1] = 1.0 + x[3] * y[3];
+    }
+    __device__ __forceinline__ static double lim_amp(const double (&r)[NLIM], int k) { return r[k]; }
+    template <class LD>
+    __device__ __forceinline__ static void lim_up(const double (&r)[NLIM], const double (&s)[MWAVES], const LD& ld,
+                                                  double (&num)[MWAVES]) {
+        const bool l0 = s[0] > 0.0, l1 = s[1] > 0.0;
+        num[0] = ld(0, l0) * (1.0 + r[2] * ld(2, l0));
+        num[1] = ld(1, l1) * (1.0 + r[3] * ld(3, l1));
+    }
+    template <int IXY>
+    __device__ __forceinline__ static void lim_sum(const Iface& f, const RPParams&, const double (&)[NLIM],
+                                                   const double (&b)[MWAVES], double (&o)[MEQN]) {
+        constexpr int MU = Dir<IXY>::MU, MV = Dir<IXY>::MV;
+        o[0] = f.zr * b[1] - f.zl * b[0];
+        o[MU] = b[0] + b[1];
+        o[MV] = 0.0;
     }
 };
 

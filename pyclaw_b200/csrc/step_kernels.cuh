@@ -41,6 +41,65 @@ struct EvolveDev {
     int cur;  // the buffer of the current state
 };
 
+// get_dt of the reference's loop (src/pyclaw/solver.py:524-552) on the loop
+// state, with Python's min/max tie rules (same values), then dt/dx, dt/dy.
+__host__ __device__ inline void evolve_get_dt(EvolveDev& e) {
+    if (e.dt_variable && e.dt_old_set) {
+        if (e.cfl > 0.0) {
+            const double x = e.dt * e.cfl_desired / e.cfl;
+            e.dt = (x < e.dt_max) ? x : e.dt_max;             // min(dt_max, x)
+            e.dtmin = (e.dtmin < e.dt) ? e.dtmin : e.dt;      // min(dt, dtmin)
+            e.dtmax = (e.dtmax > e.dt) ? e.dtmax : e.dt;      // max(dt, dtmax)
+        } else {
+            e.dt = e.dt_max;
+        }
+    } else {
+        e.dt_old_set = 1;
+    }
+    if (e.t + e.dt > e.tend && e.tstart < e.tend) e.dt = e.tend - e.t;
+    if (e.tend - e.t - e.dt < 1.e-14 * e.t) e.dt = e.tend - e.t;
+    e.dtdx = e.dt / e.dx;
+    e.dtdy = e.dt / e.dy;
+}
+
+// The end of an attempt: the reference's accept/reject (solver.py:554-666).
+// Accept when cfl <= cfl_max (t += dt, or t = tstart + (n + 1) dt with a fixed
+// dt) and make the step's buffer the current one; a rejected step keeps t and
+// the current buffer (a fixed dt ends the loop with cfl_error); the loop is
+// done when t >= tend, after max_steps attempts, or when the step produced a
+// non-finite value (fault, the step dropped); otherwise the next dt.  Returns
+// true when the next attempt starts from a new buffer, whose ghost cells are
+// still to be filled.
+__device__ __forceinline__ bool evolve_finish(EvolveDev& e, double cfl, int status) {
+    const int n = e.attempts;
+    e.attempts = n + 1;
+    e.cfl = cfl;
+    const int st = status & 3;
+    if (st) {
+        e.fault = st;
+        e.done = 1;
+        return false;
+    }
+    const bool accept = !(cfl > e.cfl_max);
+    if (accept) {
+        e.cflmax = (e.cflmax > cfl) ? e.cflmax : cfl;  // max(cfl, cflmax)
+        e.t = e.dt_variable ? __dadd_rn(e.t, e.dt) : __dadd_rn(e.tstart, __dmul_rn((double)(n + 1), e.dt));
+        e.num_steps += 1;
+        e.cur ^= 1;
+    } else if (!e.dt_variable) {
+        e.cflmax = (e.cflmax > cfl) ? e.cflmax : cfl;
+        e.cfl_error = 1;
+        e.done = 1;
+        return false;
+    }
+    if (e.t >= e.tend || e.attempts >= e.max_steps) {
+        e.done = 1;
+        return false;
+    }
+    evolve_get_dt(e);
+    return accept;
+}
+
 struct StepArgs {
     const double* __restrict__ qold;
     double* __restrict__ qnew;

@@ -65,6 +65,15 @@ struct DeviceGuard {
             return fail(CLAW2_ECUDA, "%s failed: %s", #expr, cudaGetErrorString(e_));      \
     } while (0)
 
+// Host to device, complete on return.  (cudaMemcpy from pageable memory may
+// return with its transfer to the device still under way, and work on a
+// non-blocking stream does not wait for it: the last rows of a 70001-row
+// inference were read before they had arrived.)
+cudaError_t copy_in(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 constexpr int NT_UNSPLIT = 128;  // threads per strip (124 output columns)
 constexpr int NT_SPLIT_X = 128;
 constexpr int NT_SPLIT_Y = 128;
@@ -597,10 +606,10 @@ int mlp_repack(claw2_mlp* m) {
     CUDA_TRY(cudaMemcpy(h.data(), m->P, MLP_NPARAM * 4, cudaMemcpyDeviceToHost));
     MlpPacked pk;
     mlp_pack(h.data(), pk);
-    CUDA_TRY(cudaMemcpy(m->packed, &pk, sizeof pk, cudaMemcpyHostToDevice));
+    CUDA_TRY(copy_in(m->packed, &pk, sizeof pk, m->st));
     MlpTcImage ti;
     mlp_pack_tc(h.data(), ti);
-    CUDA_TRY(cudaMemcpy(m->tc, &ti, sizeof ti, cudaMemcpyHostToDevice));
+    CUDA_TRY(copy_in(m->tc, &ti, sizeof ti, m->st));
     return CLAW2_OK;
 }
 
@@ -696,9 +705,9 @@ int claw2_mlp_create(int device, unsigned long long seed, claw2_mlp** out) {
     fill(OFF_W1, MLP_H, MLP_IN);
     fill(OFF_W2, MLP_H, MLP_H);
     fill(OFF_W3, 1, MLP_H);
-    cudaMemcpy(m->P, h.data(), MLP_NPARAM * 4, cudaMemcpyHostToDevice);
-    cudaMemset(m->M1, 0, MLP_NPARAM * 4);
-    cudaMemset(m->M2, 0, MLP_NPARAM * 4);
+    copy_in(m->P, h.data(), MLP_NPARAM * 4, m->st);
+    cudaMemsetAsync(m->M1, 0, MLP_NPARAM * 4, m->st);
+    cudaMemsetAsync(m->M2, 0, MLP_NPARAM * 4, m->st);
     int rc = mlp_repack(m);
     if (rc) {
         claw2_mlp_destroy(m);
@@ -725,7 +734,7 @@ int claw2_mlp_destroy(claw2_mlp* m) {
 int claw2_mlp_set_params(claw2_mlp* m, const float* p, int n) {
     if (!m || !p || n != MLP_NPARAM) return fail(CLAW2_EINVAL, "need %d parameters", MLP_NPARAM);
     DeviceGuard g(m->device);
-    CUDA_TRY(cudaMemcpy(m->P, p, MLP_NPARAM * 4, cudaMemcpyHostToDevice));
+    CUDA_TRY(copy_in(m->P, p, MLP_NPARAM * 4, m->st));
     return mlp_repack(m);
 }
 
@@ -819,7 +828,7 @@ int claw2_mlp_infer(claw2_mlp* m, const float* x8, int n, float* y) {
         cudaFree(dx);
         return fail(CLAW2_ENOMEM, "device allocation failed");
     }
-    cudaMemcpy(dx, x8, (size_t)n * 32, cudaMemcpyHostToDevice);
+    copy_in(dx, x8, (size_t)n * 32, m->st);
     cudaMemsetAsync(m->status, 0, 4, m->st);
     if (m->engine == CLAW2_MLP_TCGEN05)
         k_mlp_eval_tc<<<mlp_tc_grid(m, k_mlp_eval_tc, &m->eval_per_sm, (n + 255) / 256), 128, 0, m->st>>>(
@@ -2244,8 +2253,8 @@ int batch_build_tiles(claw2_batch* b, const int* rows) {
     cudaFree(b->d_tiles);
     b->d_tiles = nullptr;
     CUDA_TRY(cudaMalloc(&b->d_tiles, sizeof(int2) * b->h_tiles.size()));
-    CUDA_TRY(cudaMemcpy(b->d_tiles, b->h_tiles.data(), sizeof(int2) * b->h_tiles.size(), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(b->d_inst, b->h_inst.data(), sizeof(BatchInst) * b->n, cudaMemcpyHostToDevice));
+    CUDA_TRY(copy_in(b->d_tiles, b->h_tiles.data(), sizeof(int2) * b->h_tiles.size(), b->st));
+    CUDA_TRY(copy_in(b->d_inst, b->h_inst.data(), sizeof(BatchInst) * b->n, b->st));
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
@@ -2396,8 +2405,8 @@ int claw2_batch_create(const claw2_desc* descs, int n, claw2_batch** out) {
         claw2_batch_destroy(b);
         return fail(CLAW2_ENOMEM, "device allocation for a batch of %d instances failed", n);
     }
-    cudaMemset(b->arena, 0, total * 8);
-    cudaMemset(b->d_st, 0, sizeof(BatchState) * n);
+    cudaMemsetAsync(b->arena, 0, total * 8, b->st);
+    cudaMemsetAsync(b->d_st, 0, sizeof(BatchState) * n, b->st);
     size_t off = 0;
     for (int i = 0; i < n; ++i) {
         BatchInst& in = b->h_inst[i];
@@ -2490,7 +2499,7 @@ int claw2_batch_set_time(claw2_batch* b, const double* dt0, double t0, double te
     std::vector<BatchState> old(b->n);
     CUDA_TRY(cudaMemcpy(old.data(), b->d_st, sizeof(BatchState) * b->n, cudaMemcpyDeviceToHost));
     for (int i = 0; i < b->n; ++i) s[i].cur = old[i].cur;
-    CUDA_TRY(cudaMemcpy(b->d_st, s.data(), sizeof(BatchState) * b->n, cudaMemcpyHostToDevice));
+    CUDA_TRY(copy_in(b->d_st, s.data(), sizeof(BatchState) * b->n, b->st));
     b->ctl.cfl_desired = cfl_desired;
     b->ctl.cfl_max = cfl_max;
     b->ctl.dt_max = dt_max;

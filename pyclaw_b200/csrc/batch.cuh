@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int 
         const int strip = tl.y % in.nstrips, rblk = tl.y / in.nstrips;
         double cfl = 0.0;
         unsplit_tile<RP, NT, SPEC>(a, strip, rblk * in.H, S, cfl);
-        cfl_commit(cfl, S.red, a.cfl_bits);
+        cfl_commit(cfl, S.red, a.cfl_bits, NT / 32);
     }
 }
 

@@ -216,30 +216,44 @@ bool is_mc2(const Method& m, int mwaves) {
     return true;
 }
 
-// tm: the tensor map of qold for the TMA-staged kernel, or nullptr
+// The launch shape of a solver's unsplit step: the caller's (claw2_tune_set),
+// else three CTAs per SM, with rows staged by TMA for the solvers of four and
+// more components (the prefetch registers it frees are what spills at three CTAs:
+// 24 steps at 1024^2 Euler 2.75 -> 2.69 ms; shallow water, which does not spill,
+// 3.62 -> 3.81 ms, loads directly).  The exact solver (Newton loop and 21-number
+// record) takes two CTAs, also by TMA: six steps at 1024^2 3.94 (three, TMA) / 3.56
+// (two, direct) / 3.45 ms.
+template <class RP>
+UnsplitShape unsplit_shape() {
+    const UnsplitShape sh = g_tune[RP::ID & (TUNE_SLOTS - 1)];
+    if (sh.variant != 0 || sh.rows != 0) return {sh.variant & 3, sh.rows};
+    return {(GuessTraits<RP>::USES ? 0 : 1) | (AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
+}
+template <class RP>
+struct ShapeF {
+    static void run(UnsplitShape* sh) { *sh = unsplit_shape<RP>(); }
+};
+
+// Tiling of the unsplit kernel: strips of NT_UNSPLIT - 4 output columns,
+// row blocks of H rows (the tuned height, else the one of the least march).
+void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblocks);
+
+// tm: the tensor maps of the two buffers for the TMA-staged kernel, or nullptr
 template <class RP, int MB, int SPEC, bool EVO>
-void launch_unsplit_s(const StepArgs& b, dim3 grid, cudaStream_t st, const CUtensorMap* tm) {
-    if (!EVO && tm) {
-        constexpr int smem = (int)sizeof(UnsplitSmemTma<RP, NT_UNSPLIT>);
-        static unsigned long long attr = 0;
-        smem_attr(k_step_unsplit_tma<RP, NT_UNSPLIT, MB, SPEC>, smem, attr);
-        k_step_unsplit_tma<RP, NT_UNSPLIT, MB, SPEC><<<grid, NT_UNSPLIT, smem, st>>>(b, *tm);
-        return;
+void launch_unsplit_s(const StepArgs& b, dim3 grid, cudaStream_t st, const CUtensorMap* tm, const CUtensorMap* tm1) {
+    if constexpr (AuxTraits<RP>::MAUX == 0) {
+        if (tm) {
+            constexpr int smem = (int)sizeof(UnsplitSmemTma<RP, NT_UNSPLIT, MB>);
+            static unsigned long long attr = 0;
+            smem_attr(k_step_unsplit_tma<RP, NT_UNSPLIT, MB, SPEC, EVO>, smem, attr);
+            k_step_unsplit_tma<RP, NT_UNSPLIT, MB, SPEC, EVO><<<grid, NT_UNSPLIT, smem, st>>>(b, *tm, tm1 ? *tm1 : *tm);
+            return;
+        }
     }
     constexpr int smem = (int)sizeof(UnsplitSmem<RP, NT_UNSPLIT>);
     static unsigned long long attr = 0;
     smem_attr(k_step_unsplit<RP, NT_UNSPLIT, MB, SPEC, false, EVO>, smem, attr);
     k_step_unsplit<RP, NT_UNSPLIT, MB, SPEC, false, EVO><<<grid, NT_UNSPLIT, smem, st>>>(b);
-}
-
-// Tiling of the unsplit kernel: strips of NT_UNSPLIT - 4 output columns,
-// row blocks of H rows (the tuned height, else the heuristic).
-void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblocks) {
-    constexpr int W = NT_UNSPLIT - 4;
-    nstrips = (mx + W - 1) / W;
-    const int rows = g_tune[riemann & (TUNE_SLOTS - 1)].rows;
-    H = rows > 0 ? rows : pick_rows(nstrips, my, device_sms());
-    nblocks = (my + H - 1) / H;
 }
 
 // The capacity form (any method, rows loaded directly).
@@ -251,37 +265,37 @@ void launch_unsplit_capa(const StepArgs& b, dim3 grid, cudaStream_t st) {
     k_step_unsplit<RP, NT_UNSPLIT, 2, SPEC_ANY, true, EVO><<<grid, NT_UNSPLIT, smem, st>>>(b);
 }
 
-// EVO: a launch of the device time loop (dt read from a.evo; rows loaded
-// directly, never by TMA).
+// EVO: a launch of the device time loop (dt and buffers from a.evo).
 template <class RP, int MB, bool EVO>
-void launch_unsplit_v(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm) {
+void launch_unsplit_v(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm, const CUtensorMap* tm1) {
     StepArgs b = a;
-    int ns, H, nb;
-    unsplit_tiling(RP::ID, a.L.mx, a.L.my, ns, H, nb);
     if (b.tile_order == nullptr) {  // a caller with a schedule has fixed H and nstrips already
+        int ns, H, nb;
+        unsplit_tiling(RP::ID, a.L.mx, a.L.my, ns, H, nb);
         b.H = H;
         b.nstrips = ns;
     }
     const int nbk = (a.L.my + b.H - 1) / b.H;
     dim3 grid(b.tile_count > 0 ? b.tile_count : b.nstrips * nbk);
     if (a.capa) launch_unsplit_capa<RP, EVO>(b, grid, st);
-    else if (is_mc2(a.meth, RP::MWAVES)) launch_unsplit_s<RP, MB, SPEC_MC2, EVO>(b, grid, st, tm);
-    else launch_unsplit_s<RP, MB, SPEC_ANY, EVO>(b, grid, st, tm);
+    else if (is_mc2(a.meth, RP::MWAVES)) launch_unsplit_s<RP, MB, SPEC_MC2, EVO>(b, grid, st, tm, tm1);
+    else launch_unsplit_s<RP, MB, SPEC_ANY, EVO>(b, grid, st, tm, tm1);
 }
 
 // Variants: bit 0 = 3 blocks per SM (register cap) instead of 2, bit 1 = rows
-// staged by TMA (only where the caller has a tensor map of qold).
+// staged by TMA (only where the caller has tensor maps: of qold, or for the time
+// loop of both buffers).
 template <class RP>
-void launch_unsplit(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm) {
-    const UnsplitShape sh = g_tune[RP::ID & (TUNE_SLOTS - 1)];
+void launch_unsplit(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm, const CUtensorMap* tm1) {
+    const UnsplitShape sh = unsplit_shape<RP>();
+    const CUtensorMap* use = (sh.variant & 2) ? tm : nullptr;
     if (a.evo) {
-        if (sh.variant & 1) launch_unsplit_v<RP, 3, true>(a, st, nullptr);
-        else launch_unsplit_v<RP, 2, true>(a, st, nullptr);
+        if (sh.variant & 1) launch_unsplit_v<RP, 3, true>(a, st, use, tm1);
+        else launch_unsplit_v<RP, 2, true>(a, st, use, tm1);
         return;
     }
-    const CUtensorMap* use = (sh.variant & 2) ? tm : nullptr;
-    if (sh.variant & 1) launch_unsplit_v<RP, 3, false>(a, st, use);
-    else launch_unsplit_v<RP, 2, false>(a, st, use);
+    if (sh.variant & 1) launch_unsplit_v<RP, 3, false>(a, st, use, nullptr);
+    else launch_unsplit_v<RP, 2, false>(a, st, use, nullptr);
 }
 
 // the split sweeps' specialisation: order 2 with one limiter on every family
@@ -349,8 +363,9 @@ int dispatch(int rp, A&&... args) {
 }
 template <class RP>
 struct UnsplitF {
-    static void run(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm = nullptr) {
-        launch_unsplit<RP>(a, st, tm);
+    static void run(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm = nullptr,
+                    const CUtensorMap* tm1 = nullptr) {
+        launch_unsplit<RP>(a, st, tm, tm1);
     }
 };
 template <class RP>
@@ -359,6 +374,39 @@ struct SplitF {
         launch_split<RP>(ax, ay, st, which);
     }
 };
+
+// (declared above) The height of least march: CTAs on all slots (`per_sm` on
+// each SM) march H + 3 rows in as many waves as the tiles need, so a tile count
+// just over a multiple of the slots is a wave nearly empty (24 steps at 1024^2
+// Euler with two CTAs per SM: H = 21, 1.5 waves, 3.08 ms; 1 wave of three per SM
+// 2.75 ms).  The exact solver's tiles differ too much in their Newton work for
+// that count (one wave waits for its slowest tile: six steps at 1024^2 4.69 ms
+// against 3.45; three at 2048^2 4.58 ms with H = 64, 4.01 with 28): about three
+// blocks per SM, at most 28 rows high, taken longest first.
+void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblocks) {
+    constexpr int W = NT_UNSPLIT - 4;
+    UnsplitShape sh{0, 0};
+    dispatch<ShapeF>(riemann, &sh);
+    nstrips = (mx + W - 1) / W;
+    if (sh.rows > 0) {
+        H = sh.rows;
+    } else if (riemann == CLAW2_RP_EULER_EXACT) {
+        H = std::min(28, pick_rows(nstrips, my, device_sms()));
+    } else {
+        const long long slots = (long long)device_sms() * ((sh.variant & 1) ? 3 : 2);
+        long long best = 0;
+        H = 2;
+        for (int h = 2; h <= 64; ++h) {
+            const long long tiles = (long long)nstrips * ((my + h - 1) / h);
+            const long long rows = (tiles + slots - 1) / slots * (std::min(h, my) + 3);
+            if (best == 0 || rows < best) {
+                best = rows;
+                H = h;
+            }
+        }
+    }
+    nblocks = (my + H - 1) / H;
+}
 
 BCArgs bc_args(double* q, const Layout& L, int meqn, const int* bcl, const int* bcu, unsigned long long* cfl_bits,
                int negate, int part) {
@@ -1614,7 +1662,8 @@ int evolve_enqueue_attempt(claw2_patch* p, int c) {
             a.tile_order = p->tile_order;
             a.tile_cost = p->tile_cost;
         }
-        dispatch<UnsplitF>(p->d.riemann, a, p->st, nullptr);
+        dispatch<UnsplitF>(p->d.riemann, a, p->st, p->has_tmap ? &p->tmap[0] : nullptr,
+                           p->has_tmap ? &p->tmap[1] : nullptr);
     }
     if (lpt_n > 0 && (p->tile_steps++ % LPT_EVERY) == 0) launch_lpt(p->tile_cost, p->tile_order, lpt_n, p->st);
     const BCArgs b = bc_args(nullptr, p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, nullptr, 1, 0);

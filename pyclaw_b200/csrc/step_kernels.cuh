@@ -206,7 +206,8 @@ __device__ __forceinline__ double philim(double num, double den, int meth) {
     return neg ? 0.0 : phi;
 }
 
-__device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned long long* slot) {
+// warps: how many of the block's warps take part (the others have returned)
+__device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned long long* slot, int warps) {
     // warp max, then block max, then one 64-bit atomicMax per CTA
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cfl = fmax(cfl, __shfl_xor_sync(0xffffffffu, cfl, o));
@@ -215,7 +216,7 @@ __device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned l
     __syncthreads();
     if (threadIdx.x == 0) {
         double m = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, s_red[w]);
+        for (int w = 0; w < warps; ++w) m = fmax(m, s_red[w]);
         // non-negative doubles order like their bit patterns
         atomicMax(slot, (unsigned long long)__double_as_longlong(m));
     }
@@ -388,12 +389,18 @@ struct UnsplitSmem {
     double red[NT / 32];
 };
 
-// The TMA form's extra shared memory: the staged row (first, 128-byte
-// aligned for the copy) and its barrier.
-template <class RP, int NT>
+// Shared memory of an SM for CTAs (227 KB), and what each CTA reserves.
+constexpr int SM_SMEM = 227 * 1024, CTA_RESERVED = 1024;
+
+// The TMA form's extra shared memory: the staged rows (first, 128-byte
+// aligned for the copies) and their barriers; two rows where that leaves room
+// for MINB CTAs on an SM, so a copy has a row's work to arrive in.
+template <class RP, int NT, int MINB>
 struct UnsplitSmemTma {
-    alignas(128) double qrow[RP::MEQN][NT];
-    unsigned long long bar;
+    static constexpr int room = SM_SMEM / MINB - CTA_RESERVED - 256 - (int)sizeof(UnsplitSmem<RP, NT>);
+    static constexpr int D = room >= 2 * (int)sizeof(double) * RP::MEQN * NT ? 2 : 1;
+    alignas(128) double qrow[D][RP::MEQN][NT];
+    unsigned long long bar[D];
     UnsplitSmem<RP, NT> s;
 };
 
@@ -409,7 +416,9 @@ struct UnsplitSmemTma {
 // term of a cell carries that one factor); transverse increments carry in
 // addition the 1/kappa of the cell their fluctuation entered, the
 // second-order correction the mean of the two cells' dt/(dx kappa).
-template <class RP, int NT, int SPEC = SPEC_ANY, bool CAPA = false, bool EVO = false>
+// D: rows staged ahead.  Warps wholly past the strip's last column may have
+// returned: nothing of theirs is needed.
+template <class RP, int NT, int SPEC = SPEC_ANY, bool CAPA = false, bool EVO = false, int D = 1>
 __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int rb, UnsplitSmem<RP, NT, CAPA>& S,
                                              double& cfl, const CUtensorMap* tm = nullptr, double* qrow = nullptr,
                                              unsigned long long* bar = nullptr) {
@@ -479,9 +488,11 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
     double amY[ME], apY[ME], dY[MW];
     unsigned long long n_it = 0, n_solve = 0, n_app = 0;
     if (tma) {
-        if (t == 0) mbar_init(bar);
+        if (t == 0)
+            for (int d = 0; d < D; ++d) mbar_init(bar + d);
         __syncthreads();
-        if (t == 0) tma_row(tm, qrow, bar, x0, R0, row_bytes);
+        if (t == 0)
+            for (int d = 0; d < D && R0 + d <= R1; ++d) tma_row(tm, qrow + d * ME * NT, bar + d, x0, R0 + d, row_bytes);
     }
 #pragma unroll
     for (int m = 0; m < ME; ++m) {
@@ -505,9 +516,10 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
         {
             double q[ME], c[NC];
             if (tma) {
-                if (!mbar_wait(bar, (unsigned)(R - R0) & 1u)) atomicOr(a.status, 2);
+                const int d = (R - R0) & (D - 1);
+                if (!mbar_wait(bar + d, (unsigned)((R - R0) / D) & 1u)) atomicOr(a.status, 2);
 #pragma unroll
-                for (int m = 0; m < ME; ++m) q[m] = qrow[m * NT + tq];
+                for (int m = 0; m < ME; ++m) q[m] = qrow[(d * ME + m) * NT + tq];
             } else {
 #pragma unroll
                 for (int m = 0; m < ME; ++m) q[m] = pf[m];
@@ -532,10 +544,11 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
             }
         }
         __syncthreads();  // S1: cells of row R visible; previous exchange consumed
-        if (tma && t == 0 && R < R1) {
-            // every thread has read row R from the staging buffer (before S1)
+        if (tma && t == 0 && R + D <= R1) {
+            // every thread has read row R from its staging buffer (before S1)
+            const int d = (R - R0) & (D - 1);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            tma_row(tm, qrow, bar, x0, R + 1, row_bytes);
+            tma_row(tm, qrow + d * ME * NT, bar + d, x0, R + D, row_bytes);
         }
 
         // ---- the x-interface of row R-1, deferred transverse solve (TAUX) ----
@@ -873,21 +886,38 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
     if (GuessTraits<RP>::USES && a.counters) counter_commit(a.counters, n_it, n_solve, n_app);
 }
 
-// The same kernel with its rows staged by TMA from the tensor map of qold.
-template <class RP, int NT, int MINB, int SPEC>
-__global__ void __launch_bounds__(NT, MINB) k_step_unsplit_tma(const StepArgs a, const __grid_constant__ CUtensorMap tm) {
+// A CTA's strip, and how many of its warps have columns in the grid: the last
+// strip's warps wholly past column mx + 3 return at once (a barrier counts the
+// threads that are still there), and nothing of theirs is needed by the others.
+template <int NT>
+__device__ __forceinline__ int strip_warps(const StepArgs& a, int strip) {
+    return min(NT / 32, (a.L.mx + 4 - strip * (NT - 4) + 31) / 32);
+}
+
+__device__ __forceinline__ void tile_time(const StepArgs& a, int tile, long long t0) {
+    const long long c = clock64() - t0;
+    a.tile_cost[tile] = (unsigned int)(c < 0 ? 0 : (c > 0xffffffffll ? 0xffffffffll : c));
+}
+
+// The unsplit step with its rows staged by TMA from the tensor map of the
+// buffer it reads (tm1: of qold2, for the device time loop's launches).
+template <class RP, int NT, int MINB, int SPEC, bool EVO = false>
+__global__ void __launch_bounds__(NT, MINB) k_step_unsplit_tma(const StepArgs a, const __grid_constant__ CUtensorMap tm,
+                                                               const __grid_constant__ CUtensorMap tm1) {
+    if (EVO && a.evo->done) return;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    UnsplitSmemTma<RP, NT>& S = *reinterpret_cast<UnsplitSmemTma<RP, NT>*>(smem_raw);
-    const int tile = tile_index(a);
+    UnsplitSmemTma<RP, NT, MINB>& S = *reinterpret_cast<UnsplitSmemTma<RP, NT, MINB>*>(smem_raw);
+    const int tile = tile_index(a), strip = tile % a.nstrips;
+    const int warps = strip_warps<NT>(a, strip);
+    if ((int)(threadIdx.x >> 5) >= warps) return;
     long long t0 = 0;
     if (a.tile_cost && threadIdx.x == 0) t0 = clock64();
     double cfl = 0.0;
-    unsplit_tile<RP, NT, SPEC>(a, tile % a.nstrips, (tile / a.nstrips) * a.H, S.s, cfl, &tm, &S.qrow[0][0], &S.bar);
-    cfl_commit(cfl, S.s.red, a.cfl_bits);
-    if (a.tile_cost && threadIdx.x == 0) {
-        const long long c = clock64() - t0;
-        a.tile_cost[tile] = (unsigned int)(c < 0 ? 0 : (c > 0xffffffffll ? 0xffffffffll : c));
-    }
+    unsplit_tile<RP, NT, SPEC, false, EVO, UnsplitSmemTma<RP, NT, MINB>::D>(
+        a, strip, (tile / a.nstrips) * a.H, S.s, cfl, (EVO && a.evo->cur) ? &tm1 : &tm, &S.qrow[0][0][0],
+        &S.bar[0]);
+    cfl_commit(cfl, S.s.red, a.cfl_bits, warps);
+    if (a.tile_cost && threadIdx.x == 0) tile_time(a, tile, t0);
 }
 
 // Grid: 1D over the tiles (strip fastest).  Tile t = (strip t % nstrips, row
@@ -899,16 +929,15 @@ __global__ void __launch_bounds__(NT, MINB) k_step_unsplit(const StepArgs a) {
     if (EVO && a.evo->done) return;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     UnsplitSmem<RP, NT, CAPA>& S = *reinterpret_cast<UnsplitSmem<RP, NT, CAPA>*>(smem_raw);
-    const int tile = tile_index(a);
+    const int tile = tile_index(a), strip = tile % a.nstrips;
+    const int warps = strip_warps<NT>(a, strip);
+    if ((int)(threadIdx.x >> 5) >= warps) return;
     long long t0 = 0;
     if (a.tile_cost && threadIdx.x == 0) t0 = clock64();
     double cfl = 0.0;
-    unsplit_tile<RP, NT, SPEC, CAPA, EVO>(a, tile % a.nstrips, (tile / a.nstrips) * a.H, S, cfl);
-    cfl_commit(cfl, S.red, a.cfl_bits);
-    if (a.tile_cost && threadIdx.x == 0) {
-        const long long c = clock64() - t0;
-        a.tile_cost[tile] = (unsigned int)(c < 0 ? 0 : (c > 0xffffffffll ? 0xffffffffll : c));
-    }
+    unsplit_tile<RP, NT, SPEC, CAPA, EVO>(a, strip, (tile / a.nstrips) * a.H, S, cfl);
+    cfl_commit(cfl, S.red, a.cfl_bits, warps);
+    if (a.tile_cost && threadIdx.x == 0) tile_time(a, tile, t0);
 }
 
 // Longest-first tile schedule for the next step from this step's tile costs:
@@ -1097,7 +1126,7 @@ __global__ void __launch_bounds__(NT) k_split_x(const StepArgs a) {
             for (int m = 0; m < ME; ++m) qn[m * plane + (long long)R * pitch] = q[m];
         }
     }
-    cfl_commit(cfl, S.red, a.cfl_bits);
+    cfl_commit(cfl, S.red, a.cfl_bits, NT / 32);
 }
 
 // ---------------------------------------------------------------------------
@@ -1237,7 +1266,7 @@ __global__ void __launch_bounds__(NT) k_split_y(const StepArgs a) {
         fY = fN;
         zY = zN;
     }
-    cfl_commit(cfl, sRed, a.cfl_bits);
+    cfl_commit(cfl, sRed, a.cfl_bits, NT / 32);
 }
 
 // ---------------------------------------------------------------------------

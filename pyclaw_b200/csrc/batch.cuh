@@ -120,9 +120,10 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int 
         a.guess = nullptr;
         a.counters = nullptr;
         const int strip = tl.y % in.nstrips, rblk = tl.y / in.nstrips;
-        double cfl = 0.0;
-        unsplit_tile<RP, NT, SPEC>(a, strip, rblk * in.H, S, cfl);
-        cfl_commit(cfl, S.red, a.cfl_bits, NT / 32);
+        double sx = 0.0, sy = 0.0;
+        bool rest;
+        unsplit_tile<RP, NT, SPEC>(a, strip, rblk * in.H, S, sx, sy, rest);
+        tile_commit<false>(a, 0, S, sx, sy, rest, NT / 32);
     }
 }
 

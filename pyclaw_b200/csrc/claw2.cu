@@ -375,6 +375,11 @@ struct SplitF {
     }
 };
 
+template <class RP>
+struct KeepsRestF {
+    static void run(bool* keeps) { *keeps = KeepsRest<RP, false, true>::V; }
+};
+
 // (declared above) The height of least march: CTAs on all slots (`per_sm` on
 // each SM) march H + 3 rows in as many waves as the tiles need, so a tile count
 // just over a multiple of the slots is a wave nearly empty (24 steps at 1024^2
@@ -950,6 +955,10 @@ struct claw2_patch {
     unsigned int* tile_cost = nullptr;
     int* tile_order = nullptr;
     int tile_cap = 0, tile_n = 0, tile_H = 0;
+    // tiles at rest in the device time loop (step_kernels.cuh): two flags per tile, then the speeds
+    unsigned char* rest = nullptr;
+    double2* rest_speed = nullptr;
+    int rest_cap = 0;
     unsigned int tile_steps = 0;  // steps run on the current tiling
     long long step_launches = 0;  // kernels enqueued by patch_enqueue_step (claw2_patch_launch_count)
     // host pipeline of claw2_patch_run_host
@@ -1231,6 +1240,8 @@ int claw2_patch_destroy(claw2_patch* p) {
         for (int i = 0; i < 2; ++i)
             if (p->evo_exec[i]) cudaGraphExecDestroy(p->evo_exec[i]);
         cudaFree(p->evo);
+        cudaFree(p->rest);
+        cudaFree(p->rest_speed);
         cudaFreeHost(p->h_evo);
         cudaFree(p->cfl);
         cudaFree(p->status);
@@ -1630,10 +1641,42 @@ bool small_grid_fits(const claw2_patch* p) {
     return tiles <= 12 * p->nsm;
 }
 
+// Buffers of the at-rest flags for the marching tiles of the time loop, cleared;
+// 0 tiles (no flags) where they cannot be had, for kernels that keep none, and where the halo of a tile reaches past
+// its neighbours: row blocks of one row, or a last strip or block of one column
+// or row whose periodic images lie beyond it.
+int rest_prepare(claw2_patch* p, int ns, int H, int nb) {
+    constexpr int W = NT_UNSPLIT - 4;
+    const bool px = p->d.bc_lower[0] == CLAW2_BC_PERIODIC, py = p->d.bc_lower[1] == CLAW2_BC_PERIODIC;
+    bool keeps = false;
+    dispatch<KeepsRestF>(p->d.riemann, &keeps);
+    if (!keeps || p->d.mcapa > 0 || H < 2) return 0;
+    if ((px && p->L.mx % W == 1) || (py && p->L.my % H == 1)) return 0;
+    const int n = ns * nb;
+    if (n > p->rest_cap) {
+        cudaStreamSynchronize(p->st);
+        cudaFree(p->rest);
+        cudaFree(p->rest_speed);
+        p->rest = nullptr;
+        p->rest_speed = nullptr;
+        p->rest_cap = 0;
+        ++p->graph_gen;
+        if (cudaMalloc(&p->rest, 2 * (size_t)n) != cudaSuccess ||
+            cudaMalloc(&p->rest_speed, sizeof(double2) * n) != cudaSuccess) {
+            cudaFree(p->rest);
+            p->rest = nullptr;
+            cudaGetLastError();
+            return 0;
+        }
+        p->rest_cap = n;
+    }
+    return cudaMemsetAsync(p->rest, 0, 2 * (size_t)n, p->st) == cudaSuccess ? n : 0;
+}
+
 // One attempt of the loop with the record of parity c: step from the record's
 // current buffer into the other with its dt, then the decision, the next dt
 // and the next state's ghost cells.
-int evolve_enqueue_attempt(claw2_patch* p, int c) {
+int evolve_enqueue_attempt(claw2_patch* p, int c, int rest) {
     EvolveDev* rec = &p->evo->rec[c];
     StepArgs a = patch_args(p, 0.0);
     a.qold = p->q[0];
@@ -1661,6 +1704,12 @@ int evolve_enqueue_attempt(claw2_patch* p, int c) {
             a.nstrips = ns;
             a.tile_order = p->tile_order;
             a.tile_cost = p->tile_cost;
+        }
+        if (rest > 0) {
+            a.rest_in = p->rest + (size_t)(c ^ 1) * rest;
+            a.rest_out = p->rest + (size_t)c * rest;
+            a.rest_speed = p->rest_speed;
+            a.rest_wrap = (p->d.bc_lower[0] == CLAW2_BC_PERIODIC) | (p->d.bc_lower[1] == CLAW2_BC_PERIODIC) << 1;
         }
         dispatch<UnsplitF>(p->d.riemann, a, p->st, p->has_tmap ? &p->tmap[0] : nullptr,
                            p->has_tmap ? &p->tmap[1] : nullptr);
@@ -1790,6 +1839,12 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     CUDA_TRY(cudaMemsetAsync(p->status, 0, sizeof(int), p->st));
     bool small = small_grid_fits(p);
     if (!small) launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
+    int rest = 0;
+    if (!small && !p->d.dimensional_split) {
+        int ns, H, nb;
+        unsplit_tiling(p->d.riemann, p->L.mx, p->L.my, ns, H, nb);
+        rest = rest_prepare(p, ns, H, nb);
+    }
     long long issued = 0;
     // Attempts are issued in chunks, and the host waits for the record after
     // each.  A chunk is the number of attempts that the current dt leaves to
@@ -1849,7 +1904,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
             } else if (cudaStreamBeginCapture(p->st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
                 cudaGraph_t graph = nullptr;
                 int crc = CLAW2_OK;
-                for (int j = 0; j < GRAPH_ATTEMPTS && crc == CLAW2_OK; ++j) crc = evolve_enqueue_attempt(p, (c + j) & 1);
+                for (int j = 0; j < GRAPH_ATTEMPTS && crc == CLAW2_OK; ++j) crc = evolve_enqueue_attempt(p, (c + j) & 1, rest);
                 const cudaError_t ec = cudaStreamEndCapture(p->st, &graph);
                 if (crc != CLAW2_OK || ec != cudaSuccess || !graph ||
                     cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
@@ -1875,7 +1930,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
                     break;
                 }
         }
-        for (; chunk > 0 && rc == CLAW2_OK; --chunk, ++issued) rc = evolve_enqueue_attempt(p, (int)(issued & 1));
+        for (; chunk > 0 && rc == CLAW2_OK; --chunk, ++issued) rc = evolve_enqueue_attempt(p, (int)(issued & 1), rest);
         if (rc == CLAW2_OK) {
             if (cudaMemcpyAsync(p->h_evo, &p->evo->rec[issued & 1], sizeof(EvolveDev), cudaMemcpyDeviceToHost,
                                 p->st) != cudaSuccess ||

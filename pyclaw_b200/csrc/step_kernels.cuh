@@ -130,11 +130,50 @@ struct StepArgs {
     const EvolveDev* evo = nullptr;
     const double* qold2 = nullptr;
     double* qnew2 = nullptr;
+    // device time loop: tiles at rest (RestTiles), else nullptr
+    const unsigned char* rest_in = nullptr;
+    unsigned char* rest_out = nullptr;
+    double2* rest_speed = nullptr;
+    int rest_wrap = 0;  // bit 0 / 1: the grid is periodic in x / y
     // capacity function kappa (one plane, same layout), else nullptr: every
     // increment of a cell is divided by its kappa, a transverse increment also
     // by the kappa of the cell its fluctuation entered (step2.f90:132-160,
     // flux2.f90:104-119,134-203 with dtdx1d = dtdx / kappa)
     const double* __restrict__ capa = nullptr;
+};
+
+// Tiles at rest, in the device time loop.  A tile is at rest after an attempt
+// when every interface that attempt solved for it joined two bitwise equal cells
+// and every cell it wrote equals the one it read: its cells do not depend on dt.
+// If the eight tiles around it (which hold its halo cells and, at a boundary,
+// the sources of its ghost cells) are at rest too, the next attempt starts
+// from the same cells, and would write what both buffers already hold; only
+// its largest wave speeds are needed, for that attempt's Courant number, and
+// they are kept.  Such a tile is passed over.  The flags are kept per attempt
+// parity and cleared when a call of the loop begins, so nothing outlives it.
+// Where the flow is at rest a step costs its reads and writes and a march
+// through zero interfaces (4096^2 shallow water, four fifths at rest: 0.5 of
+// 0.6 ms); this leaves the moving part.
+__device__ __forceinline__ bool tile_rests(const unsigned char* rest, int wrap, int tx, int ty, int ntx, int nty) {
+    // (warp-collective: lane 3 j + i reads the neighbour (i - 1, j - 1); written by other SMs in the attempt before)
+    const int lane = threadIdx.x & 31;
+    bool r = true;
+    if (lane < 9) {
+        int x = tx + lane % 3 - 1, y = ty + lane / 3 - 1;
+        if (wrap & 1) x = x < 0 ? ntx - 1 : x >= ntx ? 0 : x;
+        if (wrap & 2) y = y < 0 ? nty - 1 : y >= nty ? 0 : y;
+        if (x >= 0 && x < ntx && y >= 0 && y < nty) r = __ldcg(rest + (long long)y * ntx + x) != 0;
+    }
+    return __all_sync(0xffffffffu, r);
+}
+// Which kernels keep the flags: the time loop's, for solvers of up to three
+// components.  For Euler the extra state spills at three CTAs per SM and its
+// quadrant flows leave few whole tiles at rest: 24 steps at 1024^2 2.80 ms
+// without, 3.17 ms with; shallow water 4096^2, six steps, 3.62 -> 2.63 ms (with
+// nothing at rest 5.95 -> 5.84 ms).
+template <class RP, bool CAPA, bool EVO>
+struct KeepsRest {
+    static constexpr bool V = EVO && !CAPA && RP::MEQN <= 3 && SkipTraits<RP>::OK && AuxTraits<RP>::MAUX == 0;
 };
 
 // The buffers a step reads and writes (EVO: the loop's record names them).
@@ -206,8 +245,7 @@ __device__ __forceinline__ double philim(double num, double den, int meth) {
     return neg ? 0.0 : phi;
 }
 
-// warps: how many of the block's warps take part (the others have returned)
-__device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned long long* slot, int warps) {
+__device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned long long* slot) {
     // warp max, then block max, then one 64-bit atomicMax per CTA
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cfl = fmax(cfl, __shfl_xor_sync(0xffffffffu, cfl, o));
@@ -216,7 +254,7 @@ __device__ __forceinline__ void cfl_commit(double cfl, double* s_red, unsigned l
     __syncthreads();
     if (threadIdx.x == 0) {
         double m = 0.0;
-        for (int w = 0; w < warps; ++w) m = fmax(m, s_red[w]);
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, s_red[w]);
         // non-negative doubles order like their bit patterns
         atomicMax(slot, (unsigned long long)__double_as_longlong(m));
     }
@@ -386,7 +424,8 @@ struct UnsplitSmem {
     double yr[2][ME][NT];    // increments for column cp+1: rows R-2, R-1
     double icap[CAPA ? 3 : 1][CAPA ? NT : 1];  // 1 / kappa of the ring's cells (capacity form)
     double yrec[YS ? NF + 2 * ME + MW : 1][YS ? NT : 1];  // (YS) record, A-dq, A+dq, dots of (R-2 | R-1)
-    double red[NT / 32];
+    double red[2][NT / 32];
+    int rest[NT / 32];  // per warp: its part of the tile is at rest
 };
 
 // Shared memory of an SM for CTAs (227 KB), and what each CTA reserves.
@@ -406,8 +445,10 @@ struct UnsplitSmemTma {
 
 // One tile: the strip `strip` (columns strip*W .. strip*W+NT-1, padded) and
 // the interior rows [rb, rb + H) of one grid.  Returns this thread's CFL
-// contribution in `cfl`; the caller reduces it (the tile ends with every
-// shared-memory read done, so a persistent CTA can start the next tile).
+// contribution in sx, or, in a kernel that keeps at-rest flags, its largest
+// wave speeds in sx and sy and whether its warp's part is at rest; the caller
+// reduces them (the tile ends with every shared-memory read done, so a
+// persistent CTA can start the next tile).
 // With a tensor map (tm != nullptr; qrow and bar in shared memory) the rows
 // are staged by TMA, else each thread loads its column a row ahead.
 //
@@ -420,8 +461,8 @@ struct UnsplitSmemTma {
 // returned: nothing of theirs is needed.
 template <class RP, int NT, int SPEC = SPEC_ANY, bool CAPA = false, bool EVO = false, int D = 1>
 __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int rb, UnsplitSmem<RP, NT, CAPA>& S,
-                                             double& cfl, const CUtensorMap* tm = nullptr, double* qrow = nullptr,
-                                             unsigned long long* bar = nullptr) {
+                                             double& sx, double& sy, bool& rest, const CUtensorMap* tm = nullptr,
+                                             double* qrow = nullptr, unsigned long long* bar = nullptr) {
     constexpr int ME = RP::MEQN, MW = RP::MWAVES, NC = RP::NC, W = NT - 4;
     using Iface = typename RP::Iface;
 
@@ -475,6 +516,8 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
     constexpr bool ZS = SkipTraits<RP>::OK && MA == 0 && !CAPA;
     const bool zs = ZS && (SPEC != SPEC_ANY || a.meth.fwave == 0);
     bool zY = false;  // the y-interface being finished, (R-2 | R-1), is zero in the whole warp
+    constexpr bool TRACK = KeepsRest<RP, CAPA, EVO>::V;
+    rest = TRACK && zs;
 
     // (the copy needs a 128-byte aligned destination; anything else loads
     // directly; solvers with aux data load directly)
@@ -622,6 +665,7 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
             double dn[MW];  // limiter numerators of (R-1 | R) from (R-2 | R-1), and da the other way round
             double da[MW];
             const bool zN = zs && __all_sync(0xffffffffu, same_q<ME, NC>(cB, cA));
+            if (TRACK) rest = rest && zN;
             if (ZS && zN) {
                 SkipTraits<RP>::template zero_iface<2>(cB, cA, P, fN);
 #pragma unroll
@@ -651,8 +695,10 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
             if (R >= R0 + 3) {
                 // capacity form: dt/(dy kappa) of the cells below (R-2) and above (R-1)
                 const double ydl = CAPA ? dtdy * S.icap[s0][t] : dtdy, ydr = CAPA ? dtdy * S.icap[s1][t] : dtdy;
-                if (ycfl_col)
-                    cfl = fmax(cfl, CAPA ? iface_cfl2<RP, 2>(fY, P, ydl, ydr) : iface_cfl<RP, 2>(fY, P, dtdy));
+                if (ycfl_col) {
+                    if (TRACK) sy = fmax(sy, MaxSpeed<RP>::template get<2>(fY, P));
+                    else sx = fmax(sx, CAPA ? iface_cfl2<RP, 2>(fY, P, ydl, ydr) : iface_cfl<RP, 2>(fY, P, dtdy));
+                }
             }
             if (R >= R0 + 3 && !(ZS && zY)) {
                 const double ydl = CAPA ? dtdy * S.icap[s0][t] : dtdy, ydr = CAPA ? dtdy * S.icap[s1][t] : dtdy;
@@ -764,6 +810,7 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
             }
             // (the first and last rows' x-interfaces are never finished: no solve)
             zX = ZS && (!xrow || (zs && __all_sync(0xffffffffu, same_q<ME, NC>(cL, cR))));
+            if (TRACK) rest = rest && zX;
             if (ZS && zX) {
                 SkipTraits<RP>::template zero_iface<1>(cL, cR, P, fX);
                 if (GuessTraits<RP>::USES && xrow && cp <= mx + 3 && t > 0) n_solve += 1;
@@ -792,7 +839,10 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
         if (xrow) {
             // capacity form: dt/(dx kappa) of the cells left (cp-1) and right (cp)
             const double xdl = CAPA ? dtdx * S.icap[s2][tl] : dtdx, xdr = CAPA ? dtdx * S.icap[s2][t] : dtdx;
-            if (xcfl_col) cfl = fmax(cfl, CAPA ? iface_cfl2<RP, 1>(fX, P, xdl, xdr) : iface_cfl<RP, 1>(fX, P, dtdx));
+            if (xcfl_col) {
+                if (TRACK) sx = fmax(sx, MaxSpeed<RP>::template get<1>(fX, P));
+                else sx = fmax(sx, CAPA ? iface_cfl2<RP, 1>(fX, P, xdl, xdr) : iface_cfl<RP, 1>(fX, P, dtdx));
+            }
         }
         if (xrow && !(ZS && zX)) {
             const double xdl = CAPA ? dtdx * S.icap[s2][tl] : dtdx, xdr = CAPA ? dtdx * S.icap[s2][t] : dtdx;
@@ -862,6 +912,7 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
         }
 
         // ---- row R-2 is complete ----
+        bool kept = true;  // (TRACK) the cell is written as it was read
         if (R >= R0 + 4 && out_col) {
             double v[ME];
             const double ik = CAPA ? S.icap[s0][t] : 1.0;
@@ -870,7 +921,13 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
 #pragma unroll
             for (int m = 0; m < ME; ++m) qn[m * plane + (long long)(R - 2) * pitch] = v[m];
             if (!all_finite<ME>(v)) atomicOr(a.status, 1);
+            if (TRACK && rest) {
+#pragma unroll
+                for (int m = 0; m < ME; ++m)
+                    kept = kept && __double_as_longlong(v[m]) == __double_as_longlong(S.cell[s0][m][t]);
+            }
         }
+        if (TRACK && rest) rest = __all_sync(0xffffffffu, kept);
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
             accA[m] = accB[m];
@@ -899,6 +956,62 @@ __device__ __forceinline__ void tile_time(const StepArgs& a, int tile, long long
     a.tile_cost[tile] = (unsigned int)(c < 0 ? 0 : (c > 0xffffffffll ? 0xffffffffll : c));
 }
 
+// Start of a time-loop tile: true when the tile is at rest and done with (its
+// Courant number committed by thread 0).
+__device__ __forceinline__ bool tile_passed_over(const StepArgs& a, int tile) {
+    if (!a.rest_in) return false;
+    const int nty = (a.L.my + a.H - 1) / a.H;
+    if (!tile_rests(a.rest_in, a.rest_wrap, tile % a.nstrips, tile / a.nstrips, a.nstrips, nty)) return false;
+    if (threadIdx.x == 0) {
+        const double2 s = a.rest_speed[tile];
+        const double cfl = fmax(a.evo->dtdx * s.x, a.evo->dtdy * s.y);
+        atomicMax(a.cfl_bits, (unsigned long long)__double_as_longlong(cfl));
+        a.rest_out[tile] = 1;
+        if (a.tile_cost) a.tile_cost[tile] = 0;
+    }
+    return true;
+}
+
+// End of a tile: block maximum of the CFL contributions (or of the speeds), one
+// 64-bit atomicMax of the Courant number, and (TRACK) whether the tile is at rest.
+template <bool TRACK, class S>
+__device__ __forceinline__ void tile_commit(const StepArgs& a, int tile, S& sm, double sx, double sy, bool rest,
+                                            int warps) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        sx = fmax(sx, __shfl_xor_sync(0xffffffffu, sx, o));
+        if (TRACK) sy = fmax(sy, __shfl_xor_sync(0xffffffffu, sy, o));
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        sm.red[0][warp] = sx;
+        if (TRACK) {
+            sm.red[1][warp] = sy;
+            sm.rest[warp] = rest;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double mx = 0.0, my = 0.0;
+        bool r = true;
+        for (int w = 0; w < warps; ++w) {
+            mx = fmax(mx, sm.red[0][w]);
+            if (TRACK) {
+                my = fmax(my, sm.red[1][w]);
+                r = r && sm.rest[w];
+            }
+        }
+        // (max of products = product with the max: rounding is monotonic)
+        const double cfl = TRACK ? fmax(a.evo->dtdx * mx, a.evo->dtdy * my) : mx;
+        // non-negative doubles order like their bit patterns
+        atomicMax(a.cfl_bits, (unsigned long long)__double_as_longlong(cfl));
+        if (TRACK && a.rest_out) {
+            a.rest_out[tile] = r;
+            if (r) a.rest_speed[tile] = make_double2(mx, my);
+        }
+    }
+}
+
 // The unsplit step with its rows staged by TMA from the tensor map of the
 // buffer it reads (tm1: of qold2, for the device time loop's launches).
 template <class RP, int NT, int MINB, int SPEC, bool EVO = false>
@@ -910,13 +1023,16 @@ __global__ void __launch_bounds__(NT, MINB) k_step_unsplit_tma(const StepArgs a,
     const int tile = tile_index(a), strip = tile % a.nstrips;
     const int warps = strip_warps<NT>(a, strip);
     if ((int)(threadIdx.x >> 5) >= warps) return;
+    constexpr bool TRACK = KeepsRest<RP, false, EVO>::V;
+    if (TRACK && tile_passed_over(a, tile)) return;
     long long t0 = 0;
     if (a.tile_cost && threadIdx.x == 0) t0 = clock64();
-    double cfl = 0.0;
+    double sx = 0.0, sy = 0.0;
+    bool rest;
     unsplit_tile<RP, NT, SPEC, false, EVO, UnsplitSmemTma<RP, NT, MINB>::D>(
-        a, strip, (tile / a.nstrips) * a.H, S.s, cfl, (EVO && a.evo->cur) ? &tm1 : &tm, &S.qrow[0][0][0],
+        a, strip, (tile / a.nstrips) * a.H, S.s, sx, sy, rest, (EVO && a.evo->cur) ? &tm1 : &tm, &S.qrow[0][0][0],
         &S.bar[0]);
-    cfl_commit(cfl, S.s.red, a.cfl_bits, warps);
+    tile_commit<TRACK>(a, tile, S.s, sx, sy, rest, warps);
     if (a.tile_cost && threadIdx.x == 0) tile_time(a, tile, t0);
 }
 
@@ -932,11 +1048,14 @@ __global__ void __launch_bounds__(NT, MINB) k_step_unsplit(const StepArgs a) {
     const int tile = tile_index(a), strip = tile % a.nstrips;
     const int warps = strip_warps<NT>(a, strip);
     if ((int)(threadIdx.x >> 5) >= warps) return;
+    constexpr bool TRACK = KeepsRest<RP, CAPA, EVO>::V;
+    if (TRACK && tile_passed_over(a, tile)) return;
     long long t0 = 0;
     if (a.tile_cost && threadIdx.x == 0) t0 = clock64();
-    double cfl = 0.0;
-    unsplit_tile<RP, NT, SPEC, CAPA, EVO>(a, strip, (tile / a.nstrips) * a.H, S, cfl);
-    cfl_commit(cfl, S.red, a.cfl_bits, warps);
+    double sx = 0.0, sy = 0.0;
+    bool rest;
+    unsplit_tile<RP, NT, SPEC, CAPA, EVO>(a, strip, (tile / a.nstrips) * a.H, S, sx, sy, rest);
+    tile_commit<TRACK>(a, tile, S, sx, sy, rest, warps);
     if (a.tile_cost && threadIdx.x == 0) tile_time(a, tile, t0);
 }
 
@@ -1126,7 +1245,7 @@ __global__ void __launch_bounds__(NT) k_split_x(const StepArgs a) {
             for (int m = 0; m < ME; ++m) qn[m * plane + (long long)R * pitch] = q[m];
         }
     }
-    cfl_commit(cfl, S.red, a.cfl_bits, NT / 32);
+    cfl_commit(cfl, S.red, a.cfl_bits);
 }
 
 // ---------------------------------------------------------------------------
@@ -1266,7 +1385,7 @@ __global__ void __launch_bounds__(NT) k_split_y(const StepArgs a) {
         fY = fN;
         zY = zN;
     }
-    cfl_commit(cfl, sRed, a.cfl_bits, NT / 32);
+    cfl_commit(cfl, sRed, a.cfl_bits);
 }
 
 // ---------------------------------------------------------------------------

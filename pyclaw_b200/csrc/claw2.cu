@@ -107,6 +107,7 @@ RPParams make_params(int rp, const double* cparam, int n) {
     p.flags = 0;
     if (rp == CLAW2_RP_EULER_ROE || rp == CLAW2_RP_SHALLOW_ROE || rp == CLAW2_RP_EULER_5WAVE)
         p.flags = (p.c[1] != 0.0) ? 1 : 0;
+    p.derive(rp);
     return p;
 }
 

@@ -144,6 +144,7 @@ int claw2_step2ds_noalloc(const claw2_desc* d, const double* qold, double* qnew,
     a.H = 0;
     for (int k = 0; k < CLAW2_MAX_PARAMS; ++k) a.rp.c[k] = k < d->ncparam ? d->cparam[k] : 0.0;
     a.rp.flags = (d->riemann == CLAW2_RP_EULER_ROE || d->riemann == CLAW2_RP_SHALLOW_ROE) && a.rp.c[1] != 0.0;
+    a.rp.derive(d->riemann);
     a.meth.order = d->order;
     a.meth.transverse = -1;
     a.meth.fwave = 0;

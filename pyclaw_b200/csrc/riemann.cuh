@@ -175,7 +175,7 @@ struct RPAcoustics {
         const double cc = p.c[2], zz = p.c[3];
         const double delta1 = cR[0] - cL[0];
         const double delta2 = cR[MU] - cL[MU];
-        const double i2z = rcp_nr(2.0 * zz);
+        const double i2z = p.k[0];
         const double a1 = (-delta1 + zz * delta2) * i2z;
         const double a2 = (delta1 + zz * delta2) * i2z;
         f.alpha[0] = a1;
@@ -188,7 +188,7 @@ struct RPAcoustics {
                                                 double (&bm)[MEQN], double (&bp)[MEQN]) {
         constexpr int MU = Dir<IXY>::MU, MV = Dir<IXY>::MV;
         const double cc = p.c[2], zz = p.c[3];
-        const double i2z = rcp_nr(2.0 * zz);
+        const double i2z = p.k[0];
         const double a1 = (-asdq[0] + zz * asdq[MV]) * i2z;
         const double a2 = (asdq[0] + zz * asdq[MV]) * i2z;
         bm[0] = cc * a1 * zz; bm[MU] = 0.0; bm[MV] = -cc * a1;
@@ -244,7 +244,7 @@ struct RPEulerRoe {
     struct Iface { double alpha[4]; double u, v, a, ia, H; };
 
     __device__ __forceinline__ static void prepare(const double (&q)[MEQN], const RPParams& p, double (&c)[NC]) {
-        const double gamma = p.c[0], gamma1 = gamma - 1.0;
+        const double gamma = p.c[0], gamma1 = p.c[0] - 1.0;
         const double irho = rcp_nr(q[0]);
         const double u = q[1] * irho, v = q[2] * irho;
         const double pr = gamma1 * (q[3] - 0.5 * (q[1] * u + q[2] * v));
@@ -323,7 +323,7 @@ struct RPEulerRoe {
                                                  Iface& f, double (&amdq)[MEQN], double (&apdq)[MEQN]) {
         constexpr int MU = Dir<IXY>::MU, MV = Dir<IXY>::MV;
         constexpr int UN = (IXY == 1) ? UX : UY;
-        const double gamma = p.c[0], gamma1 = gamma - 1.0;
+        const double gamma = p.c[0], gamma1 = p.c[0] - 1.0;
         roe_state<IXY>(cL, cR, p, f);
         const double u = f.u, v = f.v, H = f.H, a = f.a, ia = f.ia;
         const double u2v2 = u * u + v * v;
@@ -822,8 +822,11 @@ struct RPEulerExact {
         int applied;  // Newton steps applied: the needed ones plus the final sub-tolerance step
     };
 
+    __device__ __forceinline__ static exact_euler::Gas gas(const RPParams& p) {
+        return {p.c[0], p.k[2], p.k[3], p.k[4], p.k[5], p.k[6], p.k[7], p.k[8]};
+    }
     __device__ __forceinline__ static void prepare(const double (&q)[MEQN], const RPParams& p, double (&c)[NC]) {
-        const double gamma = p.c[0], gamma1 = gamma - 1.0;
+        const double gamma = p.c[0], gamma1 = p.k[0];
         // (k_exact_pstar_guess forms these the same way)
         const double irho = rcp_nr(q[0]);
         const double u = q[1] * irho, v = q[2] * irho;
@@ -873,7 +876,7 @@ struct RPEulerExact {
                                                    double guess, Iface& f, double (&amdq)[MEQN],
                                                    double (&apdq)[MEQN]) {
         constexpr int UN = (IXY == 1) ? UX : UY, UT = (IXY == 1) ? UY : UX;
-        const double gamma = p.c[0], gamma1 = gamma - 1.0, g1inv = 1.0 / gamma1;
+        const double gamma1 = p.k[0], g1inv = p.k[1];
         const double tol = p.c[1];
         // Roe state for the transverse solver
         {
@@ -886,7 +889,7 @@ struct RPEulerExact {
             f.ia = rsqrt_nr(a2);
             f.a = a2 * f.ia;
         }
-        const exact_euler::Gas G = exact_euler::make_gas(gamma);
+        const exact_euler::Gas G = gas(p);
         const double rl = cL[0], ul = cL[UN], vl = cL[UT], pl = cL[PP], cl = cL[CS];
         const double rr = cR[0], ur = cR[UN], vr = cR[UT], pr = cR[PP], cr = cR[CS];
         if (exact_euler::vacuum(G, ul, cl, ur, cr)) {
@@ -913,14 +916,14 @@ struct RPEulerExact {
             f.applied = 0;
             return;
         }
-        double ps, us;
+        double ps, us, xl, xr;
         int it;
-        exact_euler::star(G, rl, ul, pl, cl, rr, ur, pr, cr, guess, tol, 50, ps, us, it);
+        exact_euler::star(G, rl, ul, pl, cl, rr, ur, pr, cr, guess, tol, 50, ps, us, it, xl, xr);
         f.iters = it;
         // star() returns at once for equal states; otherwise it also applies
         // the step that falls below the tolerance (unless it stopped at its cap)
         f.applied = (rl == rr && ul == ur && pl == pr) ? 0 : (it < 50 ? it + 1 : it);
-        const exact_euler::Fan F = exact_euler::fan(G, rl, ul, pl, cl, rr, ur, pr, cr, ps, us);
+        const exact_euler::Fan F = exact_euler::fan(G, rl, ul, pl, cl, rr, ur, pr, cr, ps, us, xl, xr);
         double QL[MEQN], QR[MEQN], QsL[MEQN], QsR[MEQN];
 #pragma unroll
         for (int m = 0; m < MEQN; ++m) { QL[m] = cL[m]; QR[m] = cR[m]; }
@@ -962,7 +965,7 @@ struct RPEulerExact {
     __device__ __forceinline__ static void zero_iface(const double (&cL)[NC], const double (&cR)[NC],
                                                       const RPParams& p, Iface& f) {
         constexpr int UN = (IXY == 1) ? UX : UY;
-        const exact_euler::Gas G = exact_euler::make_gas(p.c[0]);
+        const exact_euler::Gas G = gas(p);
         const double ul = cL[UN], cl = cL[CS], ur = cR[UN], cr = cR[CS];
 #pragma unroll
         for (int k = 0; k < 3; ++k)

@@ -5,10 +5,9 @@
 // three launches, all device-side so a multi-step loop can be captured in a
 // CUDA graph with no host round trip:
 //   k_batch_bc        ghost cells of every active instance (solver.py:351-519)
-//   k_batch_step      a persistent kernel: the CTAs walk one flat work list of
-//                     (instance, strip, row block) tiles -- largest instances
-//                     first -- and run the unsplit tile of step_kernels.cuh on
-//                     each; the CFL of a tile goes to its instance's word
+//   k_batch_step      the unsplit tile of step_kernels.cuh over one flat work list
+//                     of (instance, strip, row block) tiles, largest instances
+//                     first; the CFL of a tile goes to its instance's word
 //   k_batch_finalize  per instance, the reference's accept/reject and dt rule
 //                     (solver.py:524-552, 619-651): accept swaps the q buffers,
 //                     reject keeps them; dt <- min(dt_max, dt*cfl_desired/cfl),
@@ -96,35 +95,39 @@ static __global__ void k_batch_bc(const BatchArgs b, int first, int bcl0, int bc
     }
 }
 
+// One CTA per tile, in the order of the work list (the block scheduler hands the
+// next tile to the first SM that is free). Bound by FP64 issue and the row's three
+// barriers like the step of one grid, whose blocks per SM it shares. 24 Euler problems of
+// sides 64 to 512 (2.4 M cells), ms per step: 0.348 as a persistent kernel that walked
+// the list at two blocks per SM with its old row heights; 0.264.
 template <class RP, int NT, int MINB, int SPEC>
-__global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int first, int count) {
+__global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int first) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     UnsplitSmem<RP, NT>& S = *reinterpret_cast<UnsplitSmem<RP, NT>*>(smem_raw);
-    const int end = min(first + count, b.ntiles);
-    for (int w = first + blockIdx.x; w < end; w += gridDim.x) {
-        const int2 tl = b.tiles[w];
-        const BatchInst& in = b.inst[tl.x];
-        BatchState& s = b.st[tl.x];
-        if (s.done) continue;  // uniform across the CTA
-        StepArgs a;
-        a.qold = in.q[s.cur];
-        a.qnew = in.q[s.cur ^ 1];
-        a.L = in.L;
-        a.dtdx = s.dt / in.dx;
-        a.dtdy = s.dt / in.dy;
-        a.H = in.H;
-        a.rp = b.rp;
-        a.meth = b.meth;
-        a.cfl_bits = &s.cfl_bits;
-        a.status = &s.status;
-        a.guess = nullptr;
-        a.counters = nullptr;
-        const int strip = tl.y % in.nstrips, rblk = tl.y / in.nstrips;
-        double sx = 0.0, sy = 0.0;
-        bool rest;
-        unsplit_tile<RP, NT, SPEC>(a, strip, rblk * in.H, S, sx, sy, rest);
-        tile_commit<false>(a, 0, S, sx, sy, rest, NT / 32);
-    }
+    const int2 tl = b.tiles[first + blockIdx.x];
+    const BatchInst& in = b.inst[tl.x];
+    BatchState& s = b.st[tl.x];
+    if (s.done) return;
+    StepArgs a;
+    a.qold = in.q[s.cur];
+    a.qnew = in.q[s.cur ^ 1];
+    a.L = in.L;
+    a.dtdx = s.dt / in.dx;
+    a.dtdy = s.dt / in.dy;
+    a.H = in.H;
+    a.rp = b.rp;
+    a.meth = b.meth;
+    a.cfl_bits = &s.cfl_bits;
+    a.status = &s.status;
+    a.guess = nullptr;
+    a.counters = nullptr;
+    const int strip = tl.y % in.nstrips, rblk = tl.y / in.nstrips;
+    const int warps = strip_warps<NT>(a, strip);
+    if ((int)(threadIdx.x >> 5) >= warps) return;
+    double sx = 0.0, sy = 0.0;
+    bool rest;
+    unsplit_tile<RP, NT, SPEC>(a, strip, rblk * in.H, S, sx, sy, rest);
+    tile_commit<false>(a, 0, S, sx, sy, rest, warps);
 }
 
 // one thread per instance (solver.py:524-552, 604-651)

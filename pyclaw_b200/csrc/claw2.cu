@@ -183,6 +183,12 @@ int pick_rows(int nstrips, int nrows, int nsm) {
     return std::max(2, std::min(64, H));
 }
 
+// Rows a CTA slot marches until a list of tiles of h rows is done (`rows` in all, each
+// tile's three extra rows included): its share, and on average half a tile of waiting.
+double list_march(long long rows, int slots, int h) {
+    return (double)rows / slots + 0.5 * (h + 3);
+}
+
 // ---- launches, one instantiation per Riemann solver -----------------------
 // Opt a kernel into more than 48 KB of dynamic shared memory, once per device.
 template <class K>
@@ -222,13 +228,14 @@ bool is_mc2(const Method& m, int mwaves) {
 // more components (the prefetch registers it frees are what spills at three CTAs:
 // 24 steps at 1024^2 Euler 2.75 -> 2.69 ms; shallow water, which does not spill,
 // 3.62 -> 3.81 ms, loads directly).  The exact solver (Newton loop and 21-number
-// record) takes two CTAs, also by TMA: six steps at 1024^2 3.94 (three, TMA) / 3.56
-// (two, direct) / 3.45 ms.
+// record) takes two CTAs (six steps at 1024^2 3.92 ms with three, 3.51 with two), whose
+// registers hold the next row: 2.17 ms directly, 2.20 by TMA.
 template <class RP>
 UnsplitShape unsplit_shape() {
     const UnsplitShape sh = g_tune[RP::ID & (TUNE_SLOTS - 1)];
     if (sh.variant != 0 || sh.rows != 0) return {sh.variant & 3, sh.rows};
-    return {(GuessTraits<RP>::USES ? 0 : 1) | (AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
+    if (GuessTraits<RP>::USES) return {0, 0};
+    return {1 | (AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
 }
 template <class RP>
 struct ShapeF {
@@ -387,19 +394,27 @@ struct KeepsRestF {
 // Euler with two CTAs per SM: H = 21, 1.5 waves, 3.08 ms; 1 wave of three per SM
 // 2.75 ms).  The exact solver's tiles differ too much in their Newton work for
 // that count (one wave waits for its slowest tile: six steps at 1024^2 4.69 ms
-// against 3.45; three at 2048^2 4.58 ms with H = 64, 4.01 with 28): about three
-// blocks per SM, at most 28 rows high, taken longest first.
+// against 3.45; three at 2048^2 4.58 ms with H = 64, 4.01 with 28): taken longest
+// first, their march is list_march's, and at most that of three blocks per SM.  Best
+// measured height and this one, at rows per slot of 3, 12, 31, 35, 118 and 169: 3 / 3,
+// 8 / 8, 12 / 14, 14 / 15, 32 / 27, 40 / 32, never more than 2% apart in time (28 at
+// most before: six steps at 1500 x 800 2.40 -> 2.12 ms, at 1024^2 2.38 -> 2.18 ms).
 void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblocks) {
     constexpr int W = NT_UNSPLIT - 4;
     UnsplitShape sh{0, 0};
     dispatch<ShapeF>(riemann, &sh);
     nstrips = (mx + W - 1) / W;
+    const int slots = device_sms() * ((sh.variant & 1) ? 3 : 2);
     if (sh.rows > 0) {
         H = sh.rows;
     } else if (riemann == CLAW2_RP_EULER_EXACT) {
-        H = std::min(28, pick_rows(nstrips, my, device_sms()));
+        H = 2;
+        for (int h = 3; h <= 64; ++h)
+            if (list_march((long long)nstrips * (my + 3 * ((my + h - 1) / h)), slots, h) <
+                list_march((long long)nstrips * (my + 3 * ((my + H - 1) / H)), slots, H))
+                H = h;
+        H = std::min(H, pick_rows(nstrips, my, device_sms()));
     } else {
-        const long long slots = (long long)device_sms() * ((sh.variant & 1) ? 3 : 2);
         long long best = 0;
         H = 2;
         for (int h = 2; h <= 64; ++h) {
@@ -2346,8 +2361,7 @@ constexpr int batch_blocks() {
 
 // Row-block height the instances share (each takes the equal blocks next below it).
 // The batch fills the chip as a whole, so the height follows from the rows of all
-// instances: a tile of h rows marches h + 3, the list ends on average half a tile after
-// its share per CTA, and a list that fits in one wave takes its tile, whose rows then
+// instances (list_march); a list that fits in one wave takes its tile, whose rows then
 // cost 1.2 times as much (every SM is full until the end; 4.3 against 3.6 us a row).
 // Euler, sides 64 to 512, ms per step, the measured best of 17 heights / this rule / one
 // height per instance as if it were alone (the rule before): 6 instances 0.074 / 0.074 /
@@ -2363,7 +2377,7 @@ int batch_rows(const claw2_batch* b, int slots) {
             tiles += strips * blocks;
             rows += strips * (in.L.my + 3 * blocks);
         }
-        const double cost = tiles <= slots ? 1.2 * (h + 3) : (double)rows / slots + 0.5 * (h + 3);
+        const double cost = tiles <= slots ? 1.2 * (h + 3) : list_march(rows, slots, h);
         if (h == 2 || cost < best) {
             best = cost;
             H = h;

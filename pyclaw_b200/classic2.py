@@ -56,10 +56,19 @@ def _aux(aux, rp, method):
     return a.shape[0], a
 
 
-def _prep(qold, qnew, method, mthlim):
+def _prep(qold, qnew, method, mthlim, num_ghost, mx, my, whole=False):
+    """(qold, result, method, mthlim). The step writes the result's interior (``whole``:
+    all of it), so of qnew only the ghost cells are copied (500 x 500 of four
+    components: 8 MB and 0.7 of 2.3 ms for the full copy)."""
     qold = np.asfortranarray(qold, dtype=np.float64)
     if qnew is qold:
         out = qold
+    elif num_ghost == 2 and np.shape(qnew) == qold.shape == (qold.shape[0], mx + 4, my + 4):
+        qnew = np.asarray(qnew)
+        out = np.empty(qold.shape, order='F')
+        if not whole:
+            for ghost in (np.s_[:, :, :2], np.s_[:, :, -2:], np.s_[:, :2, 2:-2], np.s_[:, -2:, 2:-2]):
+                out[ghost] = qnew[ghost]
     else:
         out = np.array(qnew, dtype=np.float64, order='F', copy=True)
     return qold, out, np.ascontiguousarray(method, dtype=np.intc), np.ascontiguousarray(mthlim, dtype=np.intc)
@@ -70,7 +79,7 @@ def step2(maxm, num_ghost, mx, my, qold, qnew, aux, dx, dy, dt, method, mthlim, 
     """Unsplit step (step2.f90); returns (qnew, cfl)."""
     rp = _solver(rpn2)
     lib = _lib.load()
-    qold, out, method, mthlim = _prep(qold, qnew, method, mthlim)
+    qold, out, method, mthlim = _prep(qold, qnew, method, mthlim, num_ghost, mx, my)
     meqn = qold.shape[0]
     cfl = np.zeros(1)
     cp = _cparam_vector(rp)
@@ -90,7 +99,7 @@ def step2ds(maxm, num_ghost, mx, my, qold, qnew, aux, dx, dy, dt, method, mthlim
     lib = _lib.load()
     if qold is qnew:
         qold = np.array(qold, dtype=np.float64, order='F', copy=True)
-    qold, out, method, mthlim = _prep(qold, qnew, method, mthlim)
+    qold, out, method, mthlim = _prep(qold, qnew, method, mthlim, num_ghost, mx, my, whole=ids == 1)
     meqn = qold.shape[0]
     cfl = np.zeros(1)
     cp = _cparam_vector(rp)

@@ -650,7 +650,9 @@ struct claw2_mlp {
     int device = 0;
     float* P = nullptr;      // parameters (FP32)
     float* G = nullptr;      // gradient (claw2_mlp_gradient)
-    float* part = nullptr;   // k_train_grad's partial sums, train_rows() rows
+    float* part = nullptr;   // the training CTAs' partial sums, train_cap() rows
+    TrainCtl* ctl = nullptr; // k_train_epoch's barrier
+    int train_per_sm = 0;    // its resident CTAs per SM (0: no cooperative launches here)
     float* M1 = nullptr;     // Adam moments
     float* M2 = nullptr;
     float* loss = nullptr;
@@ -682,7 +684,7 @@ int mlp_repack(claw2_mlp* m) {
     return CLAW2_OK;
 }
 
-// Rows of a network's partial-sum array: four CTAs of k_train_grad per SM.
+// Rows of a network's partial-sum array: four training CTAs per SM.
 int train_cap(int device) {
     int n = 0;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 148;
@@ -693,8 +695,23 @@ int train_cap(int device) {
 void mlp_batch_launch(claw2_mlp* m, long long first, int count, float* grad, float lr, int step) {
     const int rows = (int)std::min<long long>(4LL * m->nsm, ((long long)count + TRAIN_TS - 1) / TRAIN_TS);
     k_train_grad<<<rows, 256, 0, m->st>>>(m->P, m->x, m->y, m->ok, first, count, 1.f / count, m->part);
-    k_train_update<<<(TRAIN_ROW + 31) / 32, 256, 0, m->st>>>(m->part, rows, m->P, grad, m->M1, m->M2, m->loss, lr,
+    k_train_update<<<TRAIN_GROUPS, 256, 0, m->st>>>(m->part, rows, m->P, grad, m->M1, m->M2, m->loss, lr,
                                                              0.9f, 0.999f, 1e-8f, step);
+}
+
+// Minibatches [b0, b0 + nb) of an epoch's samples as one cooperative launch, `done` of
+// `total` minibatches before it.  A CTA for each tile, or for each group of the sums'
+// columns if those are more, as far as they are resident together.
+cudaError_t mlp_epoch_launch(claw2_mlp* m, long long b0, int nb, int batch, long long done, long long total, float lr) {
+    if (m->train_per_sm <= 0) return cudaErrorNotSupported;
+    const int tiles = (batch + TRAIN_TS - 1) / TRAIN_TS;
+    const int grid = std::min(std::max(tiles, TRAIN_GROUPS), std::min(4, m->train_per_sm) * m->nsm);
+    cudaError_t e = cudaMemsetAsync(m->ctl, 0, sizeof(TrainCtl), m->st);
+    if (e != cudaSuccess) return e;
+    TrainArgs a{m->P, m->x, m->y, m->ok, m->part, m->M1, m->M2, m->loss, m->ctl, done, total, b0, batch, nb,
+                m->adam_step, lr};
+    void* args[] = {&a};
+    return cudaLaunchCooperativeKernel((const void*)k_train_epoch, dim3(grid), dim3(256), args, 0, m->st);
 }
 
 // CTAs of a tcgen05 kernel: the resident ones only (each allocates TMEM once
@@ -748,7 +765,8 @@ int claw2_mlp_create(int device, unsigned long long seed, claw2_mlp** out) {
     bool ok = cudaMalloc(&m->P, MLP_NPARAM * 4) == cudaSuccess && cudaMalloc(&m->G, MLP_NPARAM * 4) == cudaSuccess &&
               cudaMalloc(&m->M1, MLP_NPARAM * 4) == cudaSuccess && cudaMalloc(&m->M2, MLP_NPARAM * 4) == cudaSuccess &&
               cudaMalloc(&m->loss, 4) == cudaSuccess &&
-              cudaMalloc(&m->part, sizeof(float) * TRAIN_ROW * train_cap(device)) == cudaSuccess && cudaMalloc(&m->packed, sizeof(MlpPacked)) == cudaSuccess &&
+              cudaMalloc(&m->part, sizeof(float) * TRAIN_ROW * train_cap(device)) == cudaSuccess &&
+              cudaMalloc(&m->ctl, sizeof(TrainCtl)) == cudaSuccess && cudaMalloc(&m->packed, sizeof(MlpPacked)) == cudaSuccess &&
               cudaMalloc(&m->tc, sizeof(MlpTcImage)) == cudaSuccess && cudaMalloc(&m->status, 4) == cudaSuccess &&
               cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) == cudaSuccess;
     if (!ok) {
@@ -758,6 +776,10 @@ int claw2_mlp_create(int device, unsigned long long seed, claw2_mlp** out) {
     }
     if (cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || m->nsm <= 0)
         m->nsm = 148;
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&m->train_per_sm, k_train_epoch, 256, 0) != cudaSuccess)
+        m->train_per_sm = 0;
     // the tcgen05 kernels' residency, found here (not inside a stream capture),
     // with the whole shared-memory carveout asked for so it is reached
     cudaFuncSetAttribute(k_mlp_guess_tc, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -792,7 +814,7 @@ int claw2_mlp_destroy(claw2_mlp* m) {
         DeviceGuard g(m->device);
         if (m->st) cudaStreamSynchronize(m->st);
         cudaFree(m->P); cudaFree(m->G); cudaFree(m->M1); cudaFree(m->M2); cudaFree(m->loss);
-        cudaFree(m->part);
+        cudaFree(m->part); cudaFree(m->ctl);
         cudaFree(m->packed); cudaFree(m->tc); cudaFree(m->status); cudaFree(m->x); cudaFree(m->y); cudaFree(m->ok);
         if (m->st) cudaStreamDestroy(m->st);
     }
@@ -874,11 +896,22 @@ int claw2_mlp_train(claw2_mlp* m, int epochs, int batch, float lr, float* last_l
     float l = 0.f;
     for (int e = 0; e < epochs; ++e) {
         CUDA_TRY(cudaMemsetAsync(m->loss, 0, 4, m->st));
-        for (long long b = 0; b < nb; ++b) {
-            ++m->adam_step;
-            // step size decays linearly to a tenth over the run
-            const float frac = (float)(e * nb + b) / (float)(epochs * nb);
-            mlp_batch_launch(m, b * batch, batch, nullptr, lr * (1.f - 0.9f * frac), m->adam_step);
+        int fault = 0;
+        for (long long b = 0; b < nb;) {
+            const int n = (int)std::min<long long>(nb - b, 4096);  // (tens of milliseconds per launch)
+            if (mlp_epoch_launch(m, b, n, batch, e * nb + b, epochs * nb, lr) == cudaSuccess) {
+                CUDA_TRY(cudaMemcpyAsync(&fault, &m->ctl->fault, 4, cudaMemcpyDeviceToHost, m->st));
+                CUDA_TRY(cudaStreamSynchronize(m->st));
+                if (fault) return fail(CLAW2_ETIMEOUT, "a barrier of the training kernel gave up");
+            } else {  // a device that refuses the cooperative launch
+                cudaGetLastError();
+                for (int k = 0; k < n; ++k) {
+                    const float frac = (float)(e * nb + b + k) / (float)(epochs * nb);
+                    mlp_batch_launch(m, (b + k) * batch, batch, nullptr, lr * (1.f - 0.9f * frac), m->adam_step + k + 1);
+                }
+            }
+            m->adam_step += n;
+            b += n;
         }
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaMemcpyAsync(&l, m->loss, 4, cudaMemcpyDeviceToHost, m->st));

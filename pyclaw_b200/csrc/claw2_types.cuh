@@ -125,4 +125,15 @@ __device__ __forceinline__ double rsqrt_nr(double x) {
     return (y == y) ? y : y0;
 }
 
+#ifdef __CUDACC__
+// For barriers over a cooperative grid: polls of the arrival count before a wait is
+// given up (each an L2 round trip: about a second in all), and the poll.
+constexpr int GRID_SPIN_LIMIT = 1 << 20;
+__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
+    unsigned int v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+#endif
+
 }  // namespace claw2

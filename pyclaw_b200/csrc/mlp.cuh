@@ -7,9 +7,11 @@
 // W2[32][32], b2[32], W3[32], b3.
 //
 // Training (all kernels of this file, FP32): k_gen_samples draws seeded
-// Riemann problems and solves each to tol by FP64 Newton; k_train_grad runs
-// forward and backward for a minibatch, leaving each CTA's gradient sums in a
-// row of a partial-sum array; k_train_update adds the rows and applies Adam.
+// Riemann problems and solves each to tol by FP64 Newton; k_train_epoch runs the
+// minibatches of an epoch: forward and backward, each CTA's gradient sums in a row
+// of a partial-sum array, then the sum of the rows and Adam.  k_train_grad and
+// k_train_update are the same two halves as launches of their own (the gradient
+// alone; devices without cooperative launches).
 //
 // Inference: k_mlp_guess_tc, one thread per grid site, evaluates the MLP for
 // the x- and y-interface of the site (interfaces with a weak jump keep the
@@ -106,11 +108,11 @@ static __global__ void k_gen_samples(unsigned long long seed, long long first, i
 // matrix product from shared memory (rows of TRAIN_LD = 68 floats: 16-byte
 // aligned, eight rows on distinct banks): 2 x 2 entries of dW2 per thread, the
 // other 290 sums one or two per thread.  They stay in registers over all tiles
-// of the CTA and go out once, as one row of `part`; k_train_update adds the rows
+// of the CTA and go out once, as one row of `part`; train_update adds the rows
 // in a fixed order, so the result does not depend on scheduling.
-// Measured per minibatch of 16384, with the update: 222 -> 19.7 us (64 of them
-// 14.3 -> 1.26 ms).  The form before, one sample per thread with a warp shuffle
-// sum per parameter, spent five shuffles and an atomic on each of 1313 numbers.
+// Measured per minibatch of 16384, with the update: 222 us with one sample per thread
+// and a warp shuffle sum per parameter (five shuffles and an atomic on each of 1313
+// numbers), 19.7 us in two launches of these tiles, 14.5 us in k_train_epoch.
 constexpr int TRAIN_TS = 64, TRAIN_LD = 68, TRAIN_ROW = MLP_NPARAM + 1;  // (a row: the gradient, then the loss)
 constexpr int TRAIN_EXTRA = OFF_W2 + (MLP_NPARAM - OFF_B2) + 1;          // sums other than dW2: 290
 
@@ -123,181 +125,303 @@ struct TrainSmem {
     float out[4][TRAIN_TS];  // output, by unit group
 };
 
+// What a thread of a training CTA reads of a tile: two numbers of one sample's features
+// (for the CTA), and its own sample's target.
+struct TrainIn {
+    float2 x;
+    float y;
+    bool act;
+};
+
+__device__ __forceinline__ TrainIn train_load(const float* __restrict__ x, const float* __restrict__ y,
+                                              const int* __restrict__ ok, long long first, int count, int t0) {
+    const int tid = threadIdx.x, s = 32 * (tid >> 7) + (tid & 31);
+    const int k = t0 + (tid >> 2), c = 2 * (tid & 3);
+    TrainIn in;
+    in.x = make_float2(0.f, 0.f);
+    if (c < MLP_IN && k < count) in.x = *reinterpret_cast<const float2*>(x + (first + k) * 8 + c);
+    in.act = t0 + s < count && ok[first + t0 + s];
+    in.y = in.act ? y[first + t0 + s] : 0.f;
+    return in;
+}
+
+// A thread's gradient sums: entries of dW2 (rows tj, tj + 16, columns ti, ti + 16), and
+// one or two of the others, each the product of two rows over the samples.
+struct TrainSums {
+    int tj, ti;
+    const float *ea[2], *eb[2];
+    float g2[2][2], ge[2];
+
+    __device__ __forceinline__ void rows_of(TrainSmem& S) {
+        const int tid = threadIdx.x;
+        tj = tid >> 4;
+        ti = tid & 15;
+        if (tid < TRAIN_LD) S.one[tid] = 1.f;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int o = tid + 256 * e;
+            ea[e] = S.one;
+            eb[e] = S.one;
+            if (o < OFF_B1) { ea[e] = S.z1[o / MLP_IN]; eb[e] = S.x[o % MLP_IN]; }
+            else if (o < OFF_W2) ea[e] = S.z1[o - OFF_B1];
+            else if (o < OFF_W2 + 32) ea[e] = S.z2[o - OFF_W2];
+            else if (o < OFF_W2 + 64) { ea[e] = S.h2[o - OFF_W2 - 32]; eb[e] = S.dy; }
+            else if (o == OFF_W2 + 64) ea[e] = S.dy;
+            else if (o == OFF_W2 + 65) ea[e] = S.loss;
+        }
+    }
+    __device__ __forceinline__ void clear() {
+        g2[0][0] = g2[0][1] = g2[1][0] = g2[1][1] = 0.f;
+        ge[0] = ge[1] = 0.f;
+    }
+    __device__ __forceinline__ void store(float* row) const {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) row[OFF_W2 + (tj + 16 * a) * MLP_H + ti + 16 * b] = g2[a][b];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int o = threadIdx.x + 256 * e;
+            if (o < TRAIN_EXTRA) row[o < OFF_W2 ? o : OFF_B2 + (o - OFF_W2)] = ge[e];
+        }
+    }
+};
+
+// Forward and backward of one tile, its sums added to R.
+__device__ __forceinline__ void train_tile(TrainSmem& S, const TrainIn& in, float inv_n, TrainSums& R) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s = 32 * (warp >> 2) + lane;  // this thread's sample of the tile
+    const int u0 = 8 * (warp & 3);          // and its units
+    __syncthreads();  // parameters in place; the last tile's sums done
+    if (2 * (tid & 3) < MLP_IN) {
+        S.x[2 * (tid & 3)][tid >> 2] = in.x.x;
+        S.x[2 * (tid & 3) + 1][tid >> 2] = in.x.y;
+    }
+    __syncthreads();
+    float h1[8], h2[8];
+    {
+        float xi[MLP_IN];
+#pragma unroll
+        for (int i = 0; i < MLP_IN; ++i) xi[i] = S.x[i][s];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float z = S.P[OFF_B1 + u0 + j];
+#pragma unroll
+            for (int i = 0; i < MLP_IN; ++i) z = fmaf(S.P[OFF_W1 + (u0 + j) * MLP_IN + i], xi[i], z);
+            h1[j] = tanhf(z);
+            S.h1[u0 + j][s] = h1[j];
+        }
+    }
+    __syncthreads();
+    {
+        float z[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) z[j] = S.P[OFF_B2 + u0 + j];
+#pragma unroll 4
+        for (int i = 0; i < MLP_H; i += 4) {
+            const float a0 = S.h1[i][s], a1 = S.h1[i + 1][s], a2 = S.h1[i + 2][s], a3 = S.h1[i + 3][s];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 w = *reinterpret_cast<const float4*>(&S.P[OFF_W2 + (u0 + j) * MLP_H + i]);
+                z[j] = fmaf(w.w, a3, fmaf(w.z, a2, fmaf(w.y, a1, fmaf(w.x, a0, z[j]))));
+            }
+        }
+        float o = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            h2[j] = tanhf(z[j]);
+            S.h2[u0 + j][s] = h2[j];
+            o = fmaf(S.P[OFF_W3 + u0 + j], h2[j], o);
+        }
+        S.out[warp & 3][s] = o;
+    }
+    __syncthreads();
+    {
+        const float o = S.P[OFF_B3] + ((S.out[0][s] + S.out[1][s]) + (S.out[2][s] + S.out[3][s]));
+        const float e = in.act ? o - in.y : 0.f, dy = e * inv_n;
+        if ((warp & 3) == 0) {
+            S.dy[s] = dy;
+            S.loss[s] = 0.5f * e * e * inv_n;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) S.z2[u0 + j][s] = dy * S.P[OFF_W3 + u0 + j] * (1.f - h2[j] * h2[j]);
+    }
+    __syncthreads();
+    {
+        float d[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d[i] = 0.f;
+#pragma unroll 8
+        for (int j = 0; j < MLP_H; ++j) {
+            const float z = S.z2[j][s];
+            const float4 wa = *reinterpret_cast<const float4*>(&S.P[OFF_W2 + j * MLP_H + u0]);
+            const float4 wb = *reinterpret_cast<const float4*>(&S.P[OFF_W2 + j * MLP_H + u0 + 4]);
+            d[0] = fmaf(wa.x, z, d[0]); d[1] = fmaf(wa.y, z, d[1]);
+            d[2] = fmaf(wa.z, z, d[2]); d[3] = fmaf(wa.w, z, d[3]);
+            d[4] = fmaf(wb.x, z, d[4]); d[5] = fmaf(wb.y, z, d[5]);
+            d[6] = fmaf(wb.z, z, d[6]); d[7] = fmaf(wb.w, z, d[7]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) S.z1[u0 + i][s] = d[i] * (1.f - h1[i] * h1[i]);
+    }
+    __syncthreads();
+    auto dot4 = [](const float4& a, const float4& b, float c) {
+        return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c))));
+    };
+#pragma unroll 4
+    for (int k = 0; k < TRAIN_TS; k += 4) {
+        const float4 a0 = *reinterpret_cast<const float4*>(&S.z2[R.tj][k]);
+        const float4 a1 = *reinterpret_cast<const float4*>(&S.z2[R.tj + 16][k]);
+        const float4 b0 = *reinterpret_cast<const float4*>(&S.h1[R.ti][k]);
+        const float4 b1 = *reinterpret_cast<const float4*>(&S.h1[R.ti + 16][k]);
+        R.g2[0][0] = dot4(a0, b0, R.g2[0][0]);
+        R.g2[0][1] = dot4(a0, b1, R.g2[0][1]);
+        R.g2[1][0] = dot4(a1, b0, R.g2[1][0]);
+        R.g2[1][1] = dot4(a1, b1, R.g2[1][1]);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        if (tid + 256 * e >= TRAIN_EXTRA) break;
+#pragma unroll 4
+        for (int k = 0; k < TRAIN_TS; k += 4)
+            R.ge[e] = dot4(*reinterpret_cast<const float4*>(R.ea[e] + k),
+                           *reinterpret_cast<const float4*>(R.eb[e] + k), R.ge[e]);
+    }
+}
+
 static __global__ void __launch_bounds__(256) k_train_grad(const float* __restrict__ P, const float* __restrict__ x,
                                                            const float* __restrict__ y, const int* __restrict__ ok,
                                                            long long first, int count, float inv_n,
                                                            float* __restrict__ part) {
     __shared__ __align__(16) TrainSmem S;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int s = 32 * (warp >> 2) + lane;  // this thread's sample of the tile
-    const int u0 = 8 * (warp & 3);          // and its units
-    const int tj = tid >> 4, ti = tid & 15; // its entries of dW2: rows tj, tj + 16, columns ti, ti + 16
-    for (int k = tid; k < MLP_NPARAM; k += 256) S.P[k] = P[k];
-    if (tid < TRAIN_LD) S.one[tid] = 1.f;
-    // the other sums: rows a . b over the samples
-    const float *ea[2], *eb[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int o = tid + 256 * e;
-        ea[e] = S.one;
-        eb[e] = S.one;
-        if (o < OFF_B1) { ea[e] = S.z1[o / MLP_IN]; eb[e] = S.x[o % MLP_IN]; }
-        else if (o < OFF_W2) ea[e] = S.z1[o - OFF_B1];
-        else if (o < OFF_W2 + 32) ea[e] = S.z2[o - OFF_W2];
-        else if (o < OFF_W2 + 64) { ea[e] = S.h2[o - OFF_W2 - 32]; eb[e] = S.dy; }
-        else if (o == OFF_W2 + 64) ea[e] = S.dy;
-        else if (o == OFF_W2 + 65) ea[e] = S.loss;
-    }
-    float g2[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, ge[2] = {0.f, 0.f};
-    for (int t0 = blockIdx.x * TRAIN_TS; t0 < count; t0 += gridDim.x * TRAIN_TS) {
-        __syncthreads();  // parameters in place; the last tile's sums done
-        {
-            const int k = t0 + (tid >> 2), c = 2 * (tid & 3);
-            if (c < MLP_IN) {
-                float2 v = make_float2(0.f, 0.f);
-                if (k < count) v = *reinterpret_cast<const float2*>(x + (first + k) * 8 + c);
-                S.x[c][tid >> 2] = v.x;
-                S.x[c + 1][tid >> 2] = v.y;
-            }
-        }
-        const bool act = t0 + s < count && ok[first + t0 + s];
-        const float ys = act ? y[first + t0 + s] : 0.f;
-        __syncthreads();
-        float h1[8], h2[8];
-        {
-            float xi[MLP_IN];
-#pragma unroll
-            for (int i = 0; i < MLP_IN; ++i) xi[i] = S.x[i][s];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float z = S.P[OFF_B1 + u0 + j];
-#pragma unroll
-                for (int i = 0; i < MLP_IN; ++i) z = fmaf(S.P[OFF_W1 + (u0 + j) * MLP_IN + i], xi[i], z);
-                h1[j] = tanhf(z);
-                S.h1[u0 + j][s] = h1[j];
-            }
-        }
-        __syncthreads();
-        {
-            float z[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) z[j] = S.P[OFF_B2 + u0 + j];
-#pragma unroll 4
-            for (int i = 0; i < MLP_H; i += 4) {
-                const float a0 = S.h1[i][s], a1 = S.h1[i + 1][s], a2 = S.h1[i + 2][s], a3 = S.h1[i + 3][s];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const float4 w = *reinterpret_cast<const float4*>(&S.P[OFF_W2 + (u0 + j) * MLP_H + i]);
-                    z[j] = fmaf(w.w, a3, fmaf(w.z, a2, fmaf(w.y, a1, fmaf(w.x, a0, z[j]))));
-                }
-            }
-            float o = 0.f;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                h2[j] = tanhf(z[j]);
-                S.h2[u0 + j][s] = h2[j];
-                o = fmaf(S.P[OFF_W3 + u0 + j], h2[j], o);
-            }
-            S.out[warp & 3][s] = o;
-        }
-        __syncthreads();
-        {
-            const float o = S.P[OFF_B3] + ((S.out[0][s] + S.out[1][s]) + (S.out[2][s] + S.out[3][s]));
-            const float e = act ? o - ys : 0.f, dy = e * inv_n;
-            if ((warp & 3) == 0) {
-                S.dy[s] = dy;
-                S.loss[s] = 0.5f * e * e * inv_n;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) S.z2[u0 + j][s] = dy * S.P[OFF_W3 + u0 + j] * (1.f - h2[j] * h2[j]);
-        }
-        __syncthreads();
-        {
-            float d[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) d[i] = 0.f;
-#pragma unroll 8
-            for (int j = 0; j < MLP_H; ++j) {
-                const float z = S.z2[j][s];
-                const float4 wa = *reinterpret_cast<const float4*>(&S.P[OFF_W2 + j * MLP_H + u0]);
-                const float4 wb = *reinterpret_cast<const float4*>(&S.P[OFF_W2 + j * MLP_H + u0 + 4]);
-                d[0] = fmaf(wa.x, z, d[0]); d[1] = fmaf(wa.y, z, d[1]);
-                d[2] = fmaf(wa.z, z, d[2]); d[3] = fmaf(wa.w, z, d[3]);
-                d[4] = fmaf(wb.x, z, d[4]); d[5] = fmaf(wb.y, z, d[5]);
-                d[6] = fmaf(wb.z, z, d[6]); d[7] = fmaf(wb.w, z, d[7]);
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) S.z1[u0 + i][s] = d[i] * (1.f - h1[i] * h1[i]);
-        }
-        __syncthreads();
-        auto dot4 = [](const float4& a, const float4& b, float c) {
-            return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c))));
-        };
-#pragma unroll 4
-        for (int k = 0; k < TRAIN_TS; k += 4) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&S.z2[tj][k]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&S.z2[tj + 16][k]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&S.h1[ti][k]);
-            const float4 b1 = *reinterpret_cast<const float4*>(&S.h1[ti + 16][k]);
-            g2[0][0] = dot4(a0, b0, g2[0][0]);
-            g2[0][1] = dot4(a0, b1, g2[0][1]);
-            g2[1][0] = dot4(a1, b0, g2[1][0]);
-            g2[1][1] = dot4(a1, b1, g2[1][1]);
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            if (tid + 256 * e >= TRAIN_EXTRA) break;
-#pragma unroll 4
-            for (int k = 0; k < TRAIN_TS; k += 4)
-                ge[e] = dot4(*reinterpret_cast<const float4*>(ea[e] + k), *reinterpret_cast<const float4*>(eb[e] + k),
-                             ge[e]);
-        }
-    }
-    float* row = part + (long long)blockIdx.x * TRAIN_ROW;
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) row[OFF_W2 + (tj + 16 * a) * MLP_H + ti + 16 * b] = g2[a][b];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int o = tid + 256 * e;
-        if (o < TRAIN_EXTRA) row[o < OFF_W2 ? o : OFF_B2 + (o - OFF_W2)] = ge[e];
-    }
+    TrainSums R;
+    R.rows_of(S);
+    R.clear();
+    for (int k = threadIdx.x; k < MLP_NPARAM; k += 256) S.P[k] = P[k];
+    for (int t0 = blockIdx.x * TRAIN_TS; t0 < count; t0 += gridDim.x * TRAIN_TS)
+        train_tile(S, train_load(x, y, ok, first, count, t0), inv_n, R);
+    R.store(part + (long long)blockIdx.x * TRAIN_ROW);
 }
 
-// Sum of the rows of `part` (in a fixed order) and, per parameter, Adam (Kingma
-// & Ba 2015) or, with grad non-null, the gradient itself; the loss is added to
-// *loss.  One CTA takes 32 columns, eight row groups side by side: the 256 rows
-// of a 16384 minibatch are 32 independent loads per thread.
-static __global__ void __launch_bounds__(256) k_train_update(const float* __restrict__ part, int rows, float* P,
-                                                             float* grad, float* m, float* v, float* loss, float lr,
-                                                             float b1, float b2, float eps, int step) {
-    __shared__ float sum[8][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int k = blockIdx.x * 32 + tx;
+// Sum of the rows of `part` (in a fixed order) over TRAIN_COLS of the columns and, per
+// parameter, Adam (Kingma & Ba 2015) or, with grad non-null, the gradient itself; the
+// loss is added to *loss.  32 row groups side by side: the 256 rows of a 16384
+// minibatch are eight independent loads per thread.
+constexpr int TRAIN_COLS = 8, TRAIN_GROUPS = (TRAIN_ROW + TRAIN_COLS - 1) / TRAIN_COLS;
+
+struct TrainSumSmem {
+    float sum[256 / TRAIN_COLS][TRAIN_COLS + 1];
+};
+
+__device__ __forceinline__ void train_update(TrainSumSmem& S, int group, const float* part, int rows, float* P,
+                                             float* grad, float* m, float* v, float* loss, float lr, float b1, float b2,
+                                             float eps, int step) {
+    const int tx = threadIdx.x % TRAIN_COLS, ty = threadIdx.x / TRAIN_COLS;
+    const int k = group * TRAIN_COLS + tx;
     float a = 0.f;
     if (k < TRAIN_ROW) {
 #pragma unroll 8
-        for (int r = ty; r < rows; r += 8) a += part[(long long)r * TRAIN_ROW + k];
+        for (int r = ty; r < rows; r += 256 / TRAIN_COLS) a += __ldcg(part + (long long)r * TRAIN_ROW + k);
     }
-    sum[ty][tx] = a;
+    S.sum[ty][tx] = a;
     __syncthreads();
-    if (ty != 0 || k >= TRAIN_ROW) return;
-    float g = 0.f;
+    if (ty == 0 && k < TRAIN_ROW) {
+        float g = 0.f;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) g += sum[r][tx];
-    if (k == MLP_NPARAM) {
-        *loss += g;
-    } else if (grad) {
-        grad[k] = g;
-    } else {
-        const float mk = b1 * m[k] + (1.f - b1) * g;
-        const float vk = b2 * v[k] + (1.f - b2) * g * g;
-        m[k] = mk;
-        v[k] = vk;
-        const float mh = mk / (1.f - powf(b1, (float)step));
-        const float vh = vk / (1.f - powf(b2, (float)step));
-        P[k] -= lr * mh / (sqrtf(vh) + eps);
+        for (int r = 0; r < 256 / TRAIN_COLS; ++r) g += S.sum[r][tx];
+        if (k == MLP_NPARAM) {
+            *loss += g;
+        } else if (grad) {
+            grad[k] = g;
+        } else {
+            const float mk = b1 * m[k] + (1.f - b1) * g;
+            const float vk = b2 * v[k] + (1.f - b2) * g * g;
+            m[k] = mk;
+            v[k] = vk;
+            const float mh = mk / (1.f - powf(b1, (float)step));
+            const float vh = vk / (1.f - powf(b2, (float)step));
+            P[k] = __ldcg(P + k) - lr * mh / (sqrtf(vh) + eps);
+        }
+    }
+}
+
+static __global__ void __launch_bounds__(256) k_train_update(const float* part, int rows, float* P, float* grad,
+                                                             float* m, float* v, float* loss, float lr, float b1,
+                                                             float b2, float eps, int step) {
+    __shared__ TrainSumSmem S;
+    train_update(S, blockIdx.x, part, rows, P, grad, m, v, loss, lr, b1, b2, eps, step);
+}
+
+// An epoch's minibatches [b0, b0 + nb) of `total` in one cooperative launch: what a
+// minibatch's two launches cost beyond their work is their start, the parameters' way
+// through memory and the first loads of the samples (19.7 us for 16384 samples, 1.26 ms
+// for 2^20; here 14.5 us and 0.93 ms): the CTAs stay, two barriers
+// per minibatch keep the halves apart (the rows before their sums, the parameters
+// before the next forward pass), and the next samples are loaded while the sums are
+// made.  What bounds it now is the chain of short phases of a tile and the barriers.
+struct TrainCtl {
+    unsigned int arrived;  // barrier arrivals so far (modulo 2^32: a wait compares the difference)
+    int fault;             // a barrier wait was given up
+};
+
+struct TrainArgs {
+    float* P;
+    const float *x, *y;
+    const int* ok;
+    float *part, *m, *v, *loss;
+    TrainCtl* ctl;
+    long long done, total;  // minibatches before this launch, and of the whole run (step size)
+    long long b0;           // first minibatch of the epoch's samples
+    int batch, nb, step0;   // samples per minibatch, minibatches, Adam steps before
+    float lr;
+};
+
+// All CTAs of the grid have arrived; false after GRID_SPIN_LIMIT polls.
+__device__ __forceinline__ bool train_barrier(TrainCtl* ctl, unsigned int target) {
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&ctl->arrived, 1u);
+        int spins = 0;
+        while ((int)(ld_acquire(&ctl->arrived) - target) < 0 && ++spins < GRID_SPIN_LIMIT) {}
+        ok = spins < GRID_SPIN_LIMIT;
+        if (!ok) ctl->fault = 1;
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
+static __global__ void __launch_bounds__(256) k_train_epoch(const TrainArgs a) {
+    __shared__ __align__(16) TrainSmem S;
+    __shared__ TrainSumSmem U;
+    const int tiles = (a.batch + TRAIN_TS - 1) / TRAIN_TS, rows = min(tiles, (int)gridDim.x);
+    const bool mine = (int)blockIdx.x < rows;
+    const float inv_n = 1.f / a.batch;
+    TrainSums R;
+    R.rows_of(S);
+    long long first = a.b0 * a.batch;
+    unsigned int target = 0;
+    TrainIn in = train_load(a.x, a.y, a.ok, first, a.batch, blockIdx.x * TRAIN_TS);
+    for (int b = 0; b < a.nb; ++b) {
+        if (mine) {
+            for (int k = threadIdx.x; k < MLP_NPARAM; k += 256) S.P[k] = __ldcg(a.P + k);
+            R.clear();
+            train_tile(S, in, inv_n, R);
+            for (int t = blockIdx.x + gridDim.x; t < tiles; t += gridDim.x)
+                train_tile(S, train_load(a.x, a.y, a.ok, first, a.batch, t * TRAIN_TS), inv_n, R);
+            R.store(a.part + (long long)blockIdx.x * TRAIN_ROW);
+        }
+        if (!train_barrier(a.ctl, target += gridDim.x)) return;
+        first += a.batch;
+        if (b + 1 < a.nb) in = train_load(a.x, a.y, a.ok, first, a.batch, blockIdx.x * TRAIN_TS);
+        // step size: linear to a tenth over the run
+        const float frac = (float)(a.done + b) / (float)a.total;
+        const float lr = a.lr * (1.f - 0.9f * frac);
+        for (int g = blockIdx.x; g < TRAIN_GROUPS; g += gridDim.x) {
+            train_update(U, g, a.part, rows, a.P, nullptr, a.m, a.v, a.loss, lr, 0.9f, 0.999f, 1e-8f, a.step0 + b + 1);
+            __syncthreads();
+        }
+        if (b + 1 < a.nb && !train_barrier(a.ctl, target += gridDim.x)) return;
     }
 }
 

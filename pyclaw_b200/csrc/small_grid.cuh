@@ -34,8 +34,6 @@ struct SmallCtl {
     int status[3];
 };
 
-constexpr int SMALL_SPIN_LIMIT = 1 << 20;  // polls of the barrier (each an L2 round trip: about a second)
-
 template <class RP, int NY>
 struct SmallSmem {
     static constexpr int NT = 32 * NY;
@@ -48,12 +46,6 @@ struct SmallSmem {
     EvolveDev e;
     int go;
 };
-
-__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 
 // 8 bytes from global to shared memory, asynchronously (waited for by copy_wait)
 __device__ __forceinline__ void copy_async(double* dst, const double* src) {
@@ -469,9 +461,9 @@ __global__ void __launch_bounds__(32 * NY, 1) k_small_evolve(const StepArgs a, c
             atomicAdd(&ctl->arrived, 1u);
             const unsigned int target = (unsigned int)(k + 1) * gridDim.x;
             int spins = 0;
-            while (ld_acquire(&ctl->arrived) < target && ++spins < SMALL_SPIN_LIMIT) {}
+            while (ld_acquire(&ctl->arrived) < target && ++spins < GRID_SPIN_LIMIT) {}
             EvolveDev& e = S.e;
-            if (spins >= SMALL_SPIN_LIMIT) {
+            if (spins >= GRID_SPIN_LIMIT) {
                 e.fault = 2;
                 e.done = 1;
             } else {

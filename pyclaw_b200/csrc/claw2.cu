@@ -1081,13 +1081,7 @@ int lpt_prepare(claw2_patch* p, int n, int H) {
 constexpr unsigned int LPT_EVERY = 4;
 
 void launch_lpt(const unsigned int* cost, int* order, int n, cudaStream_t st) {
-    int N = 1;
-    while (N < n) N <<= 1;
-    static unsigned long long attr = 0;
-    smem_attr(k_lpt_order, (int)sizeof(unsigned long long) * LPT_MAX_TILES, attr);
-    // (the sort of up to 1024 keys double-buffers its shared-memory stages)
-    const size_t smem = sizeof(unsigned long long) * (N >= 32 && N <= 1024 ? 2 * N : N);
-    k_lpt_order<<<1, 1024, smem, st>>>(cost, order, n);
+    k_lpt_order<<<(n + LPT_KEYS - 1) / LPT_KEYS, 8 * LPT_KEYS, 0, st>>>(cost, order, n);
 }
 
 StepArgs patch_args(claw2_patch* p, double dt) {

@@ -1059,70 +1059,37 @@ __global__ void __launch_bounds__(NT, MINB) k_step_unsplit(const StepArgs a) {
     if (a.tile_cost && threadIdx.x == 0) tile_time(a, tile, t0);
 }
 
-// Longest-first tile schedule for the next step from this step's tile costs:
-// one CTA sorts (cost, tile) pairs, n <= LPT_MAX_TILES, descending by cost
-// (ties: lower tile first) with a bitonic network in shared memory, and
-// writes the tile order.  The hardware starts CTAs in block order, so the
-// most expensive tiles (the developed parts of the flow; the cost pattern
-// moves slowly from step to step) start first and the cheap ones fill the
-// tail, which evens out the SMs' finishing times.  The order changes only
-// which SM runs a tile: every result is independent of it.
-constexpr int LPT_MAX_TILES = 8192;
-// Up to 1024 tiles (one key per thread): the stages whose partner is in the
-// same warp (j < 32, 40 of the 55 stages at 1024) exchange keys by shuffles,
-// the others through two alternating shared-memory buffers, one barrier each.
-static __global__ void __launch_bounds__(1024) k_lpt_order(const unsigned int* cost, int* order, int n) {
-    extern __shared__ unsigned long long keys[];
-    int N = 1;
-    while (N < n) N <<= 1;
-    if (N >= 32 && N <= (int)blockDim.x) {
-        const int i = threadIdx.x;
-        unsigned long long x = 0ull;
-        if (i < n) x = ((unsigned long long)cost[i] << 32) | (unsigned long long)(0xffffffffu - (unsigned)i);
-        int pb = 0;
-        for (int k = 2; k <= N; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                unsigned long long y;
-                if (j >= 32) {
-                    if (i < N) keys[pb * N + i] = x;
-                    __syncthreads();
-                    y = (i < N) ? keys[pb * N + (i ^ j)] : 0ull;
-                    pb ^= 1;
-                } else {
-                    y = __shfl_xor_sync(0xffffffffu, x, j);
-                }
-                // descending blocks ((i & k) == 0) keep the larger key at the
-                // lower index of the pair, ascending blocks the smaller
-                const bool keep_max = ((i & j) == 0) == ((i & k) == 0);
-                x = keep_max ? (x > y ? x : y) : (x > y ? y : x);
-            }
-        }
-        if (i < n) order[i] = (int)(0xffffffffu - (unsigned)(x & 0xffffffffull));
-        return;
-    }
-    for (int i = threadIdx.x; i < N; i += blockDim.x)
-        keys[i] = (i < n) ? (((unsigned long long)cost[i] << 32) | (unsigned long long)(0xffffffffu - (unsigned)i))
-                          : 0ull;
+// Longest-first tile schedule for the next step from this step's tile costs,
+// n <= LPT_MAX_TILES: descending by cost, ties by the lower tile.  The hardware
+// starts CTAs in block order, so the most expensive tiles (the developed parts
+// of the flow; the cost pattern moves slowly from step to step) start first and
+// the cheap ones fill the tail, which evens out the SMs' finishing times.  The
+// order changes only which SM runs a tile: every result is independent of it.
+//
+// A tile's place is the number of tiles before it, counted: n^2 comparisons, but
+// no chain of dependent stages, and spread over the chip (LPT_KEYS tiles a CTA,
+// eight threads each, four costs a read).  One CTA's bitonic sort took
+// 49 us for 2176 tiles (4096^2 shallow water, three strides a step of 250 us).
+constexpr int LPT_MAX_TILES = 8192, LPT_KEYS = 32;
+static __global__ void __launch_bounds__(8 * LPT_KEYS) k_lpt_order(const unsigned int* cost, int* order, int n) {
+    __shared__ __align__(16) unsigned int c[LPT_MAX_TILES];
+    const int n4 = (n + 3) / 4;
+    for (int i = threadIdx.x; i < 4 * n4; i += 8 * LPT_KEYS) c[i] = i < n ? cost[i] : 0u;  // (a zero past the end precedes nothing)
     __syncthreads();
-    for (int k = 2; k <= N; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < N; i += blockDim.x) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long x = keys[i], y = keys[ixj];
-                    // descending overall: blocks with (i & k) == 0 descend, the others ascend
-                    const bool swap = ((i & k) == 0) ? (x < y) : (x > y);
-                    if (swap) {
-                        keys[i] = y;
-                        keys[ixj] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
+    const int i = blockIdx.x * LPT_KEYS + (threadIdx.x >> 3);
+    const unsigned int mine = i < n ? c[i] : 0u;
+    int before = 0;
+    for (int k = threadIdx.x & 7; k < n4; k += 8) {
+        const uint4 o = reinterpret_cast<const uint4*>(c)[k];
+        const int j = 4 * k;
+        before += (o.x > mine) + (o.x == mine && j < i);
+        before += (o.y > mine) + (o.y == mine && j + 1 < i);
+        before += (o.z > mine) + (o.z == mine && j + 2 < i);
+        before += (o.w > mine) + (o.w == mine && j + 3 < i);
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        order[i] = (int)(0xffffffffu - (unsigned)(keys[i] & 0xffffffffull));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (i < n && (threadIdx.x & 7) == 0) order[before] = i;
 }
 
 static __global__ void k_iota(int* a, int n) {

@@ -329,7 +329,7 @@ int claw2_step2ds_noalloc(const claw2_desc* desc, const double* qold, double* qn
 /* ---- batches of independent problems (the batched form) ------------------
  * n problems of different sizes with the same solver, method, BCs and
  * parameters (the unsplit step), each with its own dt and time.  One batch
- * step = ghost fill of every instance + one persistent kernel over a flat
+ * step = ghost fill of every instance + one kernel over a flat
  * list of (instance, strip, row block) tiles + a per-instance accept/reject
  * and dt update on the device (solver.py:524-552, 619-651).  Replaces a host
  * loop of ClawSolver2D.evolve_to_time calls, one per problem. */
@@ -353,7 +353,8 @@ int claw2_batch_run(claw2_batch* b, int nsteps, int mode, float* ms);
  * instance retired at its last good state (the others go on). */
 int claw2_batch_get_state(claw2_batch* b, double* t, double* dt, int* nsteps, int* nreject, double* cfl_last,
                           int* status);
-int claw2_batch_tiles(claw2_batch* b, int* ntiles, int* persistent_grid);
+/* Tiles of one batch step, and how many of them the device runs at once. */
+int claw2_batch_tiles(claw2_batch* b, int* ntiles, int* resident);
 
 /* ---- the exact Euler solver's learned Newton guess (no reference counterpart)
  * A 6-32-32-1 tanh network predicting log(p_star / p_pvrs) / w from the normalised

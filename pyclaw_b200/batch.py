@@ -3,7 +3,7 @@
 A user of the reference runs many independent problems as a host loop of
 ``Controller.run()`` / ``Solver.evolve_to_time`` calls, one problem at a time
 (src/pyclaw/solver.py:554-666).  ``Batch`` steps all of them at once: every
-batch step is one ghost-fill launch, one persistent step kernel over the tiles
+batch step is one ghost-fill launch, one step kernel over the tiles
 of all problems and one per-problem accept/reject + dt update, all on the
 device, and a run of many steps is one CUDA graph launch (claw2_batch_* in
 include/claw2.h).  Each problem keeps the reference's own dt rule

@@ -2485,7 +2485,7 @@ struct BatchOccF {
     }
 };
 
-// One batched step: ghost fill of every instance, the persistent step, finalize.
+// One batched step: ghost fill of every instance, the step over all tiles, finalize.
 void batch_step_all(claw2_batch* b) {
     const BatchArgs a = batch_args(b);
     int maxg = 0;
@@ -2738,10 +2738,10 @@ int claw2_batch_get_state(claw2_batch* b, double* t, double* dt, int* nsteps, in
     return CLAW2_OK;
 }
 
-int claw2_batch_tiles(claw2_batch* b, int* ntiles, int* persistent_grid) {
-    if (!b || !ntiles || !persistent_grid) return fail(CLAW2_EINVAL, "bad arguments");
+int claw2_batch_tiles(claw2_batch* b, int* ntiles, int* resident) {
+    if (!b || !ntiles || !resident) return fail(CLAW2_EINVAL, "bad arguments");
     *ntiles = (int)b->h_tiles.size();
-    *persistent_grid = b->resident_ctas;
+    *resident = b->resident_ctas;
     return CLAW2_OK;
 }
 

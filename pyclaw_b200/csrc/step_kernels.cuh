@@ -447,8 +447,7 @@ struct UnsplitSmemTma {
 // the interior rows [rb, rb + H) of one grid.  Returns this thread's CFL
 // contribution in sx, or, in a kernel that keeps at-rest flags, its largest
 // wave speeds in sx and sy and whether its warp's part is at rest; the caller
-// reduces them (the tile ends with every shared-memory read done, so a
-// persistent CTA can start the next tile).
+// reduces them (tile_commit).
 // With a tensor map (tm != nullptr; qrow and bar in shared memory) the rows
 // are staged by TMA, else each thread loads its column a row ahead.
 //

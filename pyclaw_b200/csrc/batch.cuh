@@ -25,7 +25,8 @@ struct BatchInst {       // static per-instance data
     double* q[2];        // ping-pong planes
     Layout L;
     double dx, dy;
-    int nstrips, H;      // tiling of this instance
+    int nstrips, H;      // tiling of this instance in the batch's step
+    int alone;           // its row height in a step of its own (BatchArgs::tiles not used)
 };
 
 struct BatchState {      // dynamic per-instance data
@@ -95,16 +96,16 @@ static __global__ void k_batch_bc(const BatchArgs b, int first, int bcl0, int bc
     }
 }
 
-// One CTA per tile, in the order of the work list (the block scheduler hands the
+// One CTA per tile (one: of that instance alone), in the order of the work list (the block scheduler hands the
 // next tile to the first SM that is free). Bound by FP64 issue and the row's three
 // barriers like the step of one grid, whose blocks per SM it shares. 24 Euler problems of
 // sides 64 to 512 (2.4 M cells), ms per step: 0.348 as a persistent kernel that walked
 // the list at two blocks per SM with its old row heights; 0.264.
 template <class RP, int NT, int MINB, int SPEC>
-__global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int first) {
+__global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int one) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     UnsplitSmem<RP, NT>& S = *reinterpret_cast<UnsplitSmem<RP, NT>*>(smem_raw);
-    const int2 tl = b.tiles[first + blockIdx.x];
+    const int2 tl = one < 0 ? b.tiles[blockIdx.x] : make_int2(one, (int)blockIdx.x);
     const BatchInst& in = b.inst[tl.x];
     BatchState& s = b.st[tl.x];
     if (s.done) return;
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int 
     a.L = in.L;
     a.dtdx = s.dt / in.dx;
     a.dtdy = s.dt / in.dy;
-    a.H = in.H;
+    a.H = one < 0 ? in.H : in.alone;
     a.rp = b.rp;
     a.meth = b.meth;
     a.cfl_bits = &s.cfl_bits;
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int 
     if ((int)(threadIdx.x >> 5) >= warps) return;
     double sx = 0.0, sy = 0.0;
     bool rest;
-    unsplit_tile<RP, NT, SPEC>(a, strip, rblk * in.H, S, sx, sy, rest);
+    unsplit_tile<RP, NT, SPEC>(a, strip, rblk * a.H, S, sx, sy, rest);
     tile_commit<false>(a, 0, S, sx, sy, rest, warps);
 }
 

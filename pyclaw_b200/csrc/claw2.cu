@@ -2360,7 +2360,6 @@ struct claw2_batch {
     std::vector<claw2_desc> descs;
     std::vector<BatchInst> h_inst;
     std::vector<int> order;          // instances by decreasing size
-    std::vector<int> tile_first, tile_count;
     std::vector<int2> h_tiles;
     BatchInst* d_inst = nullptr;
     BatchState* d_st = nullptr;
@@ -2415,21 +2414,20 @@ int batch_rows(const claw2_batch* b, int slots) {
 
 int batch_build_tiles(claw2_batch* b, const int* rows) {
     constexpr int W = NT_UNSPLIT - 4;
+    DeviceGuard g(b->device);
     b->h_tiles.clear();
-    b->tile_first.assign(b->n, 0);
-    b->tile_count.assign(b->n, 0);
     const int common = batch_rows(b, b->resident_ctas);
     for (int i : b->order) {
         BatchInst& in = b->h_inst[i];
         in.nstrips = (in.L.mx + W - 1) / W;
         const int even = (in.L.my + common - 1) / common;
         in.H = (rows && rows[i] > 0) ? rows[i] : (in.L.my + even - 1) / even;
+        // (alone on the chip it needs more, shorter tiles: 512 problems of sides 64 to 512
+        // one by one, 20 ms a step; 98 ms with the batch's heights)
+        in.alone = (rows && rows[i] > 0) ? rows[i] : pick_rows(in.nstrips, in.L.my, device_sms());
         const int nblk = (in.L.my + in.H - 1) / in.H;
-        b->tile_first[i] = (int)b->h_tiles.size();
-        b->tile_count[i] = in.nstrips * nblk;
         for (int k = 0; k < in.nstrips * nblk; ++k) b->h_tiles.push_back(make_int2(i, k));
     }
-    DeviceGuard g(b->device);
     cudaFree(b->d_tiles);
     b->d_tiles = nullptr;
     CUDA_TRY(cudaMalloc(&b->d_tiles, sizeof(int2) * b->h_tiles.size()));
@@ -2469,10 +2467,10 @@ int batch_smem_attr() {
 
 template <class RP>
 struct BatchStepF {
-    static void run(const BatchArgs& a, int first, int count, cudaStream_t st) {
+    static void run(const BatchArgs& a, int one, int count, cudaStream_t st) {
         constexpr int smem = (int)sizeof(UnsplitSmem<RP, NT_UNSPLIT>), MB = batch_blocks<RP>();
-        if (is_mc2(a.meth, RP::MWAVES)) k_batch_step<RP, NT_UNSPLIT, MB, SPEC_MC2><<<count, NT_UNSPLIT, smem, st>>>(a, first);
-        else k_batch_step<RP, NT_UNSPLIT, MB, SPEC_ANY><<<count, NT_UNSPLIT, smem, st>>>(a, first);
+        if (is_mc2(a.meth, RP::MWAVES)) k_batch_step<RP, NT_UNSPLIT, MB, SPEC_MC2><<<count, NT_UNSPLIT, smem, st>>>(a, one);
+        else k_batch_step<RP, NT_UNSPLIT, MB, SPEC_ANY><<<count, NT_UNSPLIT, smem, st>>>(a, one);
     }
 };
 
@@ -2493,7 +2491,7 @@ void batch_step_all(claw2_batch* b) {
     dim3 gbc((maxg + 255) / 256, b->n);
     k_batch_bc<<<gbc, 256, 0, b->st>>>(a, 0, b->d0.bc_lower[0], b->d0.bc_lower[1], b->d0.bc_upper[0],
                                       b->d0.bc_upper[1], b->d0.num_eqn);
-    dispatch<BatchStepF>(b->d0.riemann, a, 0, a.ntiles, b->st);
+    dispatch<BatchStepF>(b->d0.riemann, a, -1, a.ntiles, b->st);
     k_batch_finalize<<<(b->n + 127) / 128, 128, 0, b->st>>>(a, 0, b->n);
 }
 
@@ -2506,7 +2504,7 @@ void batch_step_each(claw2_batch* b) {
         k_batch_bc<<<dim3((ng + 255) / 256, 1), 256, 0, b->st>>>(a, i, b->d0.bc_lower[0], b->d0.bc_lower[1],
                                                                  b->d0.bc_upper[0], b->d0.bc_upper[1],
                                                                  b->d0.num_eqn);
-        dispatch<BatchStepF>(b->d0.riemann, a, b->tile_first[i], b->tile_count[i], b->st);
+        dispatch<BatchStepF>(b->d0.riemann, a, i, in.nstrips * ((in.L.my + in.alone - 1) / in.alone), b->st);
         k_batch_finalize<<<1, 32, 0, b->st>>>(a, i, 1);
     }
 }

@@ -230,16 +230,19 @@ bool is_mc2(const Method& m, int mwaves) {
 // 3.62 -> 3.81 ms, loads directly).  The exact solver (Newton loop and 21-number
 // record) takes two CTAs (six steps at 1024^2 3.92 ms with three, 3.51 with two), whose
 // registers hold the next row: 2.17 ms directly, 2.20 by TMA.
+// (That is the time loop's kernel.  The ordinary step, with dt in its parameters, spills as
+// much with staged rows as without, and loads directly: 1024^2 Euler, L2 flushed, H = 18
+// 0.101 ms staged, 0.090 ms direct.)
 template <class RP>
-UnsplitShape unsplit_shape() {
+UnsplitShape unsplit_shape(bool evo) {
     const UnsplitShape sh = g_tune[RP::ID & (TUNE_SLOTS - 1)];
     if (sh.variant != 0 || sh.rows != 0) return {sh.variant & 3, sh.rows};
     if (GuessTraits<RP>::USES) return {0, 0};
-    return {1 | (AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
+    return {1 | (evo && AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
 }
 template <class RP>
 struct ShapeF {
-    static void run(UnsplitShape* sh) { *sh = unsplit_shape<RP>(); }
+    static void run(UnsplitShape* sh) { *sh = unsplit_shape<RP>(false); }  // (blocks per SM and rows: the same in both)
 };
 
 // Tiling of the unsplit kernel: strips of NT_UNSPLIT - 4 output columns,
@@ -295,7 +298,7 @@ void launch_unsplit_v(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm,
 // loop of both buffers).
 template <class RP>
 void launch_unsplit(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm, const CUtensorMap* tm1) {
-    const UnsplitShape sh = unsplit_shape<RP>();
+    const UnsplitShape sh = unsplit_shape<RP>(a.evo != nullptr);
     const CUtensorMap* use = (sh.variant & 2) ? tm : nullptr;
     if (a.evo) {
         if (sh.variant & 1) launch_unsplit_v<RP, 3, true>(a, st, use, tm1);

@@ -100,7 +100,8 @@ static __global__ void k_batch_bc(const BatchArgs b, int first, int bcl0, int bc
 // next tile to the first SM that is free). Bound by FP64 issue and the row's three
 // barriers like the step of one grid, whose blocks per SM it shares. 24 Euler problems of
 // sides 64 to 512 (2.4 M cells), ms per step: 0.348 as a persistent kernel that walked
-// the list at two blocks per SM with its old row heights; 0.264.
+// the list at two blocks per SM with its old row heights; 0.249; 0.235 with its rows
+// asked for five rows early (see unsplit_tile).
 template <class RP, int NT, int MINB, int SPEC>
 __global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int one) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_step(const BatchArgs b, int 
     if ((int)(threadIdx.x >> 5) >= warps) return;
     double sx = 0.0, sy = 0.0;
     bool rest;
-    unsplit_tile<RP, NT, SPEC>(a, strip, rblk * a.H, S, sx, sy, rest);
+    unsplit_tile<RP, NT, SPEC, false, false, 1, 5>(a, strip, rblk * a.H, S, sx, sy, rest);
     tile_commit<false>(a, 0, S, sx, sy, rest, warps);
 }
 

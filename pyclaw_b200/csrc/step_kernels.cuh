@@ -443,6 +443,10 @@ struct UnsplitSmemTma {
     UnsplitSmem<RP, NT> s;
 };
 
+__device__ __forceinline__ void prefetch_l2(const double* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // One tile: the strip `strip` (columns strip*W .. strip*W+NT-1, padded) and
 // the interior rows [rb, rb + H) of one grid.  Returns this thread's CFL
 // contribution in sx, or, in a kernel that keeps at-rest flags, its largest
@@ -458,7 +462,13 @@ struct UnsplitSmemTma {
 // second-order correction the mean of the two cells' dt/(dx kappa).
 // D: rows staged ahead.  Warps wholly past the strip's last column may have
 // returned: nothing of theirs is needed.
-template <class RP, int NT, int SPEC = SPEC_ANY, bool CAPA = false, bool EVO = false, int D = 1>
+// AHEAD > 0: directly loaded rows are asked for that many rows early into L2 (one thread
+// in four: a 32-byte sector).  A row of zero jumps marches in less time than DRAM answers,
+// and a batch's planes do not stay in L2: 24 Euler problems 0.249 -> 0.235 ms per step, 60
+// 0.558 -> 0.502.  A single grid's step has no such wait, and loses to the spills (84 B
+// more) what is there to win: 24 steps at 1024^2 3.43 -> 4.03 ms, shallow water
+// 4096^2 2.55 -> 2.60 ms; for the batched step only.
+template <class RP, int NT, int SPEC = SPEC_ANY, bool CAPA = false, bool EVO = false, int D = 1, int AHEAD = 0>
 __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int rb, UnsplitSmem<RP, NT, CAPA>& S,
                                              double& sx, double& sy, bool& rest, const CUtensorMap* tm = nullptr,
                                              double* qrow = nullptr, unsigned long long* bar = nullptr) {
@@ -568,6 +578,10 @@ __device__ __forceinline__ void unsplit_tile(const StepArgs& a, int strip, int r
                 if (R < R1) {
 #pragma unroll
                     for (int m = 0; m < ME; ++m) pf[m] = __ldg(qo + m * plane + (long long)(R + 1) * pitch);
+                }
+                if (AHEAD > 0 && R + AHEAD <= R1 && (t & 3) == 0) {
+#pragma unroll
+                    for (int m = 0; m < ME; ++m) prefetch_l2(qo + m * plane + (long long)(R + AHEAD) * pitch);
                 }
             }
             double av[MAD];

@@ -41,6 +41,8 @@ WORKLOAD = "euler_quadrants_roe_1024x1024_unsplit_trans_cor_mc"
 # One ncu capture of the step kernel on this workload (profiles/k_step_unsplit_euler_roe_1024.md):
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, and the FP64 pipe's busy fraction.
 # The launch's 33.5 MB of output stays in L2 while it runs, so DRAM shows the reads only.
+# (Captured at three blocks per SM, H = 16, before the eigenvector coordinates: the bytes are the
+# same in every shape, the pipe's share moves with the shape.)
 NCU_TRAFFIC_BYTES = {1024: 34.801e6 + 0.926e6}
 NCU_FP64_PIPE_ACTIVE = {1024: 0.435}
 

@@ -223,8 +223,19 @@ bool is_mc2(const Method& m, int mwaves) {
     return true;
 }
 
+// CTAs of a solver's unsplit tile that an SM's shared memory holds, at most three
+// (what the register caps are compiled for).
+template <class RP>
+constexpr int unsplit_fit() {
+    constexpr int n = SM_SMEM / ((int)sizeof(UnsplitSmem<RP, NT_UNSPLIT>) + CTA_RESERVED);
+    static_assert(n >= 2, "two tiles must fit on an SM");
+    return n < 3 ? n : 3;
+}
+
 // The launch shape of a solver's unsplit step: the caller's (claw2_tune_set),
-// else three CTAs per SM, with rows staged by TMA for the solvers of four and
+// else three CTAs per SM where their shared memory fits (the five-component Euler solver's
+// does not: two, whose registers hold everything; 24 problems of a batch 461 -> 309 us a
+// step), with rows staged by TMA for the solvers of four and
 // more components (the prefetch registers it frees are what spills at three CTAs:
 // 24 steps at 1024^2 Euler 2.75 -> 2.69 ms; shallow water, which does not spill,
 // 3.62 -> 3.81 ms, loads directly).  The exact solver (Newton loop and 21-number
@@ -237,17 +248,13 @@ template <class RP>
 UnsplitShape unsplit_shape(bool evo) {
     const UnsplitShape sh = g_tune[RP::ID & (TUNE_SLOTS - 1)];
     if (sh.variant != 0 || sh.rows != 0) return {sh.variant & 3, sh.rows};
-    if (GuessTraits<RP>::USES) return {0, 0};
+    if (GuessTraits<RP>::USES || unsplit_fit<RP>() < 3) return {0, 0};
     return {1 | (evo && AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
 }
-template <class RP>
-struct ShapeF {
-    static void run(UnsplitShape* sh) { *sh = unsplit_shape<RP>(false); }  // (blocks per SM and rows: the same in both)
-};
 
 // Tiling of the unsplit kernel: strips of NT_UNSPLIT - 4 output columns,
 // row blocks of H rows (the tuned height, else the one of the least march).
-void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblocks);
+void unsplit_tiling(int riemann, bool capa, bool evo, int mx, int my, int& nstrips, int& H, int& nblocks);
 
 // tm: the tensor maps of the two buffers for the TMA-staged kernel, or nullptr
 template <class RP, int MB, int SPEC, bool EVO>
@@ -276,13 +283,59 @@ void launch_unsplit_capa(const StepArgs& b, dim3 grid, cudaStream_t st) {
     k_step_unsplit<RP, NT_UNSPLIT, 2, SPEC_ANY, true, EVO><<<grid, NT_UNSPLIT, smem, st>>>(b);
 }
 
+// CTAs of a step kernel that an SM runs at once: its occupancy, which registers or
+// shared memory bound.  The tiling counts waves of this many: a count that is not there
+// is a wave half empty (three counted where two ran: capacity-form Euler at 600 x 515
+// 72.6 -> 52.1 us, five-component Euler at 1000 x 858 189 -> 106 us together with the cap
+// of unsplit_shape), one that is too low leaves slots idle (advection, five CTAs per SM,
+// order 1 at 2000 x 1715 47 -> 37 us).
+template <class RP, bool EVO>
+int unsplit_resident(int variant, bool capa) {
+    static std::atomic<int> cache[5];  // by variant; the capacity form
+    std::atomic<int>& c = cache[capa ? 4 : variant];
+    int n = c.load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    auto count = [&n](auto kernel, int smem) {
+        unsigned long long attr = 0;
+        smem_attr(kernel, smem, attr);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, NT_UNSPLIT, smem) != cudaSuccess) n = 0;
+    };
+    if (capa) {
+        count(k_step_unsplit<RP, NT_UNSPLIT, 2, SPEC_ANY, true, EVO>, (int)sizeof(UnsplitSmem<RP, NT_UNSPLIT, true>));
+    } else {
+        if constexpr (AuxTraits<RP>::MAUX == 0) {
+            if (variant == 2) count(k_step_unsplit_tma<RP, NT_UNSPLIT, 2, SPEC_ANY, EVO>, (int)sizeof(UnsplitSmemTma<RP, NT_UNSPLIT, 2>));
+            if (variant == 3) count(k_step_unsplit_tma<RP, NT_UNSPLIT, 3, SPEC_ANY, EVO>, (int)sizeof(UnsplitSmemTma<RP, NT_UNSPLIT, 3>));
+        } else {
+            variant &= 1;  // (rows of solvers with aux data are loaded directly)
+        }
+        if (variant == 0) count(k_step_unsplit<RP, NT_UNSPLIT, 2, SPEC_ANY, false, EVO>, (int)sizeof(UnsplitSmem<RP, NT_UNSPLIT>));
+        if (variant == 1) count(k_step_unsplit<RP, NT_UNSPLIT, 3, SPEC_ANY, false, EVO>, (int)sizeof(UnsplitSmem<RP, NT_UNSPLIT>));
+    }
+    if (n <= 0) {
+        cudaGetLastError();
+        return 2;
+    }
+    c.store(n, std::memory_order_relaxed);
+    return n;
+}
+
+template <class RP>
+struct ShapeF {
+    static void run(bool capa, bool evo, int* rows, int* per_sm) {
+        const UnsplitShape sh = unsplit_shape<RP>(evo);
+        *rows = sh.rows;
+        *per_sm = evo ? unsplit_resident<RP, true>(sh.variant, capa) : unsplit_resident<RP, false>(sh.variant, capa);
+    }
+};
+
 // EVO: a launch of the device time loop (dt and buffers from a.evo).
 template <class RP, int MB, bool EVO>
 void launch_unsplit_v(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm, const CUtensorMap* tm1) {
     StepArgs b = a;
     if (b.tile_order == nullptr) {  // a caller with a schedule has fixed H and nstrips already
         int ns, H, nb;
-        unsplit_tiling(RP::ID, a.L.mx, a.L.my, ns, H, nb);
+        unsplit_tiling(RP::ID, a.capa != nullptr, EVO, a.L.mx, a.L.my, ns, H, nb);
         b.H = H;
         b.nstrips = ns;
     }
@@ -402,14 +455,14 @@ struct KeepsRestF {
 // measured height and this one, at rows per slot of 3, 12, 31, 35, 118 and 169: 3 / 3,
 // 8 / 8, 12 / 14, 14 / 15, 32 / 27, 40 / 32, never more than 2% apart in time (28 at
 // most before: six steps at 1500 x 800 2.40 -> 2.12 ms, at 1024^2 2.38 -> 2.18 ms).
-void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblocks) {
+void unsplit_tiling(int riemann, bool capa, bool evo, int mx, int my, int& nstrips, int& H, int& nblocks) {
     constexpr int W = NT_UNSPLIT - 4;
-    UnsplitShape sh{0, 0};
-    dispatch<ShapeF>(riemann, &sh);
+    int rows = 0, per_sm = 2;
+    dispatch<ShapeF>(riemann, capa, evo, &rows, &per_sm);
     nstrips = (mx + W - 1) / W;
-    const int slots = device_sms() * ((sh.variant & 1) ? 3 : 2);
-    if (sh.rows > 0) {
-        H = sh.rows;
+    const int slots = device_sms() * per_sm;
+    if (rows > 0) {
+        H = rows;
     } else if (riemann == CLAW2_RP_EULER_EXACT) {
         H = 2;
         for (int h = 3; h <= 64; ++h)
@@ -422,9 +475,9 @@ void unsplit_tiling(int riemann, int mx, int my, int& nstrips, int& H, int& nblo
         H = 2;
         for (int h = 2; h <= 64; ++h) {
             const long long tiles = (long long)nstrips * ((my + h - 1) / h);
-            const long long rows = (tiles + slots - 1) / slots * (std::min(h, my) + 3);
-            if (best == 0 || rows < best) {
-                best = rows;
+            const long long march = (tiles + slots - 1) / slots * (std::min(h, my) + 3);
+            if (best == 0 || march < best) {
+                best = march;
                 H = h;
             }
         }
@@ -1500,7 +1553,7 @@ namespace {
 int patch_enqueue_step(claw2_patch* p, double dt, int part = 0) {
     double* qc = p->q[p->cur];
     int ns = 0, H = 0, nb = 0;
-    unsplit_tiling(p->d.riemann, p->L.mx, p->L.my, ns, H, nb);
+    unsplit_tiling(p->d.riemann, p->d.mcapa > 0, false, p->L.mx, p->L.my, ns, H, nb);
     // row block b reads padded rows H b .. H b + min(H, my - H b) + 3: blocks
     // 1 .. b_hi read no ghost row (H (b+1) + 3 <= my + 1 for a full block;
     // a ragged last block of one row pushes its neighbour into the edge set)
@@ -1743,7 +1796,7 @@ int evolve_enqueue_attempt(claw2_patch* p, int c, int rest) {
         dispatch<SplitF>(p->d.riemann, ax, ay, p->st, 3);
     } else {
         int ns, H, nb;
-        unsplit_tiling(p->d.riemann, p->L.mx, p->L.my, ns, H, nb);
+        unsplit_tiling(p->d.riemann, p->d.mcapa > 0, true, p->L.mx, p->L.my, ns, H, nb);
         if (ns * nb > 2 * p->nsm && lpt_prepare(p, ns * nb, H) == CLAW2_OK) {
             lpt_n = ns * nb;
             a.H = H;
@@ -1888,7 +1941,7 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     int rest = 0;
     if (!small && !p->d.dimensional_split) {
         int ns, H, nb;
-        unsplit_tiling(p->d.riemann, p->L.mx, p->L.my, ns, H, nb);
+        unsplit_tiling(p->d.riemann, p->d.mcapa > 0, true, p->L.mx, p->L.my, ns, H, nb);
         rest = rest_prepare(p, ns, H, nb);
     }
     long long issued = 0;
@@ -2385,7 +2438,7 @@ namespace {
 // Blocks per SM of the batched step (see unsplit_shape).
 template <class RP>
 constexpr int batch_blocks() {
-    return GuessTraits<RP>::USES ? 2 : 3;
+    return GuessTraits<RP>::USES ? 2 : unsplit_fit<RP>();
 }
 
 // Row-block height the instances share (each takes the equal blocks next below it).

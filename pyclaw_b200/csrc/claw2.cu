@@ -1712,32 +1712,41 @@ struct SmallF {
 };
 template <class RP>
 struct SmallTilesF {
-    static void run(int mx, int my, int* tiles) {
+    static void run(int mx, int my, int* tiles, bool* half) {
         if constexpr (!GuessTraits<RP>::USES)
             *tiles = ((mx + 27) / 28) * ((my + SmallF<RP>::NY - 5) / (SmallF<RP>::NY - 4));
         else *tiles = -1;  // (a guess per interface: marching kernels only)
+        *half = SmallF<RP>::NY < 16;
     }
 };
 
 // Whether the time loop of a patch runs as the small-grid kernel.  Measured per
-// step, marching kernels against it (acoustics / shallow water / Euler, MC):
-// split, 200^2 17.4 -> 8.0 / 20.3 -> 8.9 / 21.6 -> 9.9 us, 800^2 37.6 -> 27 / 51 -> 38 /
-// 78 -> 54 us and 2500^2 273 -> 204 / 317 -> 260 / 572 -> 407 us: always.  Unsplit,
-// 200^2 15.0 -> 8.3 / 18.7 -> 9.7 / 23.3 -> 11 us, 800^2 35 -> 36 / 49 -> 40 / 83 -> 72 us,
-// 1600^2 about 95 -> 126 / 140 -> 131 / 230 -> 233 us: while the tiles are at most a
-// dozen per SM (750^2), since a tile computes its halo rows again and a
-// marching strip does not.
+// step, marching kernels with today's shapes against it, MC (acoustics / shallow water /
+// Euler).  Split: 300 x 258 18.8 -> 6.5 / 22.8 -> 9.1 / 31.3 -> 11.5 us, 1000 x 858
+// 44.8 -> 29.8 / 67.5 -> 53.0 / 102.5 -> 72.5 us, 2000 x 1715 171 -> 108 / 246 -> 199 /
+// 367 -> 275 us (the least gain, the p-system's, 299 -> 291 us): always.  Unsplit:
+// 300 x 258 18.1 -> 7.8 / 24.2 -> 10.9 / 28.9 -> 14.3 us, 600 x 515 24.3 -> 18.6 / 35.7 ->
+// 29.5 / 45.7 -> 40.8 us, 1000 x 858 41.2 against 41.9 / 67.4 against 69.7 / 93.8 against
+// 98.6 us, 2000 x 1715 118 against 156 / 204 against 261 / 294 against 372 us: while the
+// tiles are at most a dozen per SM (750^2), since a tile computes its halo rows
+// again and a marching strip does not.
+// A record that leaves room for 8 rows only (five-component Euler) writes 28 x 4 of its
+// 32 x 8 cells and gives way sooner.  Split: 300 x 258 (4.8 tiles per SM) 31.4 -> 17.2 us,
+// 550 x 472 (15.9) 54.8 -> 47.2 us, 600 x 515 (19) 55.0 against 58.2 us, 2000 x 1715 405 against 578 us.
+// Unsplit, MC and minmod: 300 x 258 27.8 -> 21.6 and 34.4 -> 30.4 us, 350 x 300 (6.6)
+// 33.4 -> 28.7 and 38.5 against 40.8 us, 450 x 386 (11) 39.5 against 46.6 and 49.6 against 65.8 us.
 bool small_grid_fits(const claw2_patch* p) {
     if (p->d.mcapa > 0) return false;  // the capacity form has no small-grid tile
     for (int d = 0; d < 2; ++d)
         if (p->d.bc_lower[d] == CLAW2_BC_NONE || p->d.bc_upper[d] == CLAW2_BC_NONE) return false;
     int tiles = -1;
-    dispatch<SmallTilesF>(p->d.riemann, p->d.mx, p->d.my, &tiles);
+    bool half = false;
+    dispatch<SmallTilesF>(p->d.riemann, p->d.mx, p->d.my, &tiles, &half);
     if (tiles < 0) return false;
-    if (p->d.dimensional_split) return true;
+    if (p->d.dimensional_split) return !half || tiles <= 16 * p->nsm;
     const UnsplitShape sh = g_tune[p->d.riemann & (TUNE_SLOTS - 1)];
     if (sh.variant != 0 || sh.rows != 0) return false;  // the caller asked for a marching shape
-    return tiles <= 12 * p->nsm;
+    return tiles <= (half ? 7 : 12) * p->nsm;
 }
 
 // Buffers of the at-rest flags for the marching tiles of the time loop, cleared;

@@ -1749,6 +1749,15 @@ bool small_grid_fits(const claw2_patch* p) {
     return tiles <= (half ? 7 : 12) * p->nsm;
 }
 
+// Attempts of one launch of the small-grid loop: about 20 ms of them, since the launch holds
+// every SM and other streams' kernels wait for its end (1024 attempts of a 2500^2 split Euler
+// run were 0.42 s, of 16384^2 18 s).  0.1 ns per cell, 5 us at the least, is a little more
+// than the slowest solver takes; the next launch costs 15 us.
+int small_grid_budget(const claw2_patch* p) {
+    const double attempt = std::max(5e-6, 1e-10 * (double)p->L.mx * p->L.my);
+    return (int)std::max(1.0, std::min(1024.0, 0.02 / attempt));
+}
+
 // Buffers of the at-rest flags for the marching tiles of the time loop, cleared;
 // 0 tiles (no flags) where they cannot be had, for kernels that keep none, and where the halo of a tile reaches past
 // its neighbours: row blocks of one row, or a last strip or block of one column
@@ -1979,7 +1988,6 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     int rc = CLAW2_OK;
     for (;;) {
         if (small) {  // the whole loop in one launch (again after a budget of attempts)
-            constexpr int BUDGET = 1024;
             cudaError_t er = cudaMemsetAsync(&p->evo->ctl, 0, sizeof(SmallCtl), p->st);
             if (er == cudaSuccess) {
                 StepArgs a = patch_args(p, 0.0);
@@ -1987,10 +1995,10 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
                 a.qnew = p->q[1];
                 a.qold2 = p->q[1];
                 const BCArgs b = bc_args(nullptr, p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, nullptr, 1, 0);
-                dispatch<SmallF>(p->d.riemann, a, b, p->evo, BUDGET, p->d.dimensional_split != 0, p->nsm, p->st, &er);
+                dispatch<SmallF>(p->d.riemann, a, b, p->evo, small_grid_budget(p), p->d.dimensional_split != 0, p->nsm, p->st, &er);
             }
             if (er == cudaSuccess) {
-                issued += 2 * BUDGET;
+                issued += 2;  // (the record stays the first: the launch writes its end into rec[0])
                 chunk = 0;
             } else if (issued > 0) {
                 rc = fail(CLAW2_ECUDA, "the small-grid loop could not continue: %s", cudaGetErrorString(er));

@@ -207,6 +207,13 @@ typedef struct claw2_evolve_state {
 } claw2_evolve_state;
 int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s);
 
+/* The time loop of a split step, and of an unsplit one on a small grid, runs
+ * as one cooperative kernel that holds every SM.  on = 1 keeps this patch's
+ * loop on the marching kernels instead, a few launches per attempt between
+ * which other streams' kernels run; it is also the loop of a device that
+ * refuses cooperative launches.  0 (default): whichever is faster. */
+int claw2_patch_set_marching(claw2_patch* p, int on);
+
 /* One hyperbolic step from the current q: ghost fill on the device, then the
  * unsplit (or split) step into the pending buffer.  If cfl is non-NULL the
  * call waits and returns the Courant number; with NULL it only enqueues. */

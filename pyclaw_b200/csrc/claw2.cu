@@ -1064,6 +1064,7 @@ struct claw2_patch {
     unsigned char* rest = nullptr;
     double2* rest_speed = nullptr;
     int rest_cap = 0;
+    bool marching = false;        // the time loop runs as marching kernels at every size (claw2_patch_set_marching)
     unsigned int tile_steps = 0;  // steps run on the current tiling
     long long step_launches = 0;  // kernels enqueued by patch_enqueue_step (claw2_patch_launch_count)
     // host pipeline of claw2_patch_run_host
@@ -1736,6 +1737,7 @@ struct SmallTilesF {
 // Unsplit, MC and minmod: 300 x 258 27.8 -> 21.6 and 34.4 -> 30.4 us, 350 x 300 (6.6)
 // 33.4 -> 28.7 and 38.5 against 40.8 us, 450 x 386 (11) 39.5 against 46.6 and 49.6 against 65.8 us.
 bool small_grid_fits(const claw2_patch* p) {
+    if (p->marching) return false;
     if (p->d.mcapa > 0) return false;  // the capacity form has no small-grid tile
     for (int d = 0; d < 2; ++d)
         if (p->d.bc_lower[d] == CLAW2_BC_NONE || p->d.bc_upper[d] == CLAW2_BC_NONE) return false;
@@ -1955,13 +1957,15 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
     CUDA_TRY(cudaMemcpyAsync(&p->evo->rec[0], p->h_evo, sizeof(EvolveDev), cudaMemcpyHostToDevice, p->st));
     CUDA_TRY(cudaMemsetAsync(p->status, 0, sizeof(int), p->st));
     bool small = small_grid_fits(p);
-    if (!small) launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
     int rest = 0;
-    if (!small && !p->d.dimensional_split) {
+    auto begin_marching = [&] {  // ghost cells of the current buffer, a clear Courant word, no tile known to rest
+        launch_bc(p->q[e.cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
+        if (p->d.dimensional_split) return;
         int ns, H, nb;
         unsplit_tiling(p->d.riemann, p->d.mcapa > 0, true, p->L.mx, p->L.my, ns, H, nb);
         rest = rest_prepare(p, ns, H, nb);
-    }
+    };
+    if (!small) begin_marching();
     long long issued = 0;
     // Attempts are issued in chunks, and the host waits for the record after
     // each.  A chunk is the number of attempts that the current dt leaves to
@@ -2000,13 +2004,11 @@ int claw2_patch_evolve(claw2_patch* p, claw2_evolve_state* s) {
             if (er == cudaSuccess) {
                 issued += 2;  // (the record stays the first: the launch writes its end into rec[0])
                 chunk = 0;
-            } else if (issued > 0) {
-                rc = fail(CLAW2_ECUDA, "the small-grid loop could not continue: %s", cudaGetErrorString(er));
-                chunk = 0;
-            } else {  // no cooperative launch to be had: the marching kernels
+            } else {  // no cooperative launch to be had (any more): the marching kernels, from the record as it is
                 cudaGetLastError();
                 small = false;
-                launch_bc(p->q[p->cur], p->L, p->d.num_eqn, p->d.bc_lower, p->d.bc_upper, &p->evo->cfl[0], p->st);
+                issued = 0;
+                begin_marching();
             }
         }
         if (issued > 0 && chunk >= GRAPH_ATTEMPTS && (issued & 1) != exec_parity) exec = nullptr;
@@ -2190,6 +2192,12 @@ int claw2_patch_sync(claw2_patch* p) {
         cudaMemsetAsync(p->status, 0, sizeof(int), p->st);
         return fail(CLAW2_ENONFINITE, "a step produced a non-finite value");
     }
+    return CLAW2_OK;
+}
+
+int claw2_patch_set_marching(claw2_patch* p, int on) {
+    if (!p) return fail(CLAW2_EINVAL, "null patch");
+    p->marching = on != 0;
     return CLAW2_OK;
 }
 

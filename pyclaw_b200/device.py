@@ -160,6 +160,10 @@ class DevicePatch(object):
             self.device_newer = True
         return rc
 
+    def set_marching(self, on):
+        """Keep the time loop on the marching kernels (claw2_patch_set_marching)."""
+        _lib.check(self._lib.claw2_patch_set_marching(self.h, 1 if on else 0))
+
     def accept(self, accept):
         _lib.check(self._lib.claw2_patch_accept(self.h, 1 if accept else 0))
         if accept:

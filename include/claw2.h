@@ -279,8 +279,14 @@ int claw2_patch_launch_count(claw2_patch* p, long long* n);
  * compiles for 2 blocks per SM (no register cap), 1 for 3 blocks per SM,
  * 2 and 3 the same with rows staged by TMA (4 and 8, two earlier tiles, are
  * accepted and run variant 0); rows = row-block height (0 = heuristic).
- * Process-wide; set by an autotuner (pyclaw_b200.tune) or by hand. */
+ * variant 0 with rows 0 takes the shape back: the library's own choice of
+ * both.  A shape set here holds for the device time loop too, and keeps an
+ * unsplit one on the marching kernels at every size; claw2_tune_set_step's is
+ * for the ordinary step alone (what an autotuner that times that step knows
+ * about).  Each replaces the other's.  Process-wide; set by an autotuner
+ * (pyclaw_b200.tune) or by hand. */
 int claw2_tune_set(int riemann, int variant, int rows);
+int claw2_tune_set_step(int riemann, int variant, int rows);
 int claw2_tune_get(int riemann, int* variant, int* rows);
 
 /* FP64 FMA throughput of the current device, TFLOP/s (2 flops per FMA): a

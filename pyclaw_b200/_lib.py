@@ -119,6 +119,7 @@ _SIGNATURES = {
     "claw2_selftest_lpt": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_ulonglong,
                                           ctypes.POINTER(ctypes.c_int)]),
     "claw2_tune_set": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
+    "claw2_tune_set_step": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "claw2_tune_get": (ctypes.c_int, [ctypes.c_int, _c_int_p, _c_int_p]),
     "claw2_step2ds_noalloc": (ctypes.c_int, [ctypes.POINTER(Claw2Desc), ctypes.c_void_p, ctypes.c_void_p,
                                              ctypes.c_longlong, ctypes.c_longlong, ctypes.c_double, _c_double_p,

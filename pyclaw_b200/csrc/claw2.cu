@@ -215,6 +215,18 @@ constexpr int TUNE_SLOTS = 16;  // indexed by Riemann solver id
 UnsplitShape g_tune[TUNE_SLOTS] = {};
 std::atomic<unsigned> g_tune_gen{0};  // bumped by every claw2_tune_set (cached graphs go stale)
 
+// The caller's shape for a solver's ordinary step or (loop) its device time loop; {0, 0}:
+// none.  A shape of claw2_tune_set_step was measured on the ordinary step, which is another
+// kernel than the loop's, and says nothing about the cooperative loop of small grids: the
+// loop keeps its own (200^2 acoustics with a shape tuned for 1024^2 15.0 us a step, 8.3 without).
+constexpr int TUNE_STEP_ONLY = 16;
+UnsplitShape tuned_shape(int riemann, bool loop) {
+    UnsplitShape sh = g_tune[riemann & (TUNE_SLOTS - 1)];
+    if (loop && (sh.variant & TUNE_STEP_ONLY)) return {0, 0};
+    sh.variant &= ~TUNE_STEP_ONLY;
+    return sh;
+}
+
 // true for the method the SPEC_MC2 kernels are compiled for
 bool is_mc2(const Method& m, int mwaves) {
     if (m.order != 2 || m.transverse != 2 || m.fwave != 0) return false;
@@ -246,7 +258,7 @@ constexpr int unsplit_fit() {
 // 0.101 ms staged, 0.090 ms direct.)
 template <class RP>
 UnsplitShape unsplit_shape(bool evo) {
-    const UnsplitShape sh = g_tune[RP::ID & (TUNE_SLOTS - 1)];
+    const UnsplitShape sh = tuned_shape(RP::ID, evo);
     if (sh.variant != 0 || sh.rows != 0) return {sh.variant & 3, sh.rows};
     if (GuessTraits<RP>::USES || unsplit_fit<RP>() < 3) return {0, 0};
     return {1 | (evo && AuxTraits<RP>::MAUX == 0 && RP::MEQN >= 4 ? 2 : 0), 0};
@@ -1746,7 +1758,7 @@ bool small_grid_fits(const claw2_patch* p) {
     dispatch<SmallTilesF>(p->d.riemann, p->d.mx, p->d.my, &tiles, &half);
     if (tiles < 0) return false;
     if (p->d.dimensional_split) return !half || tiles <= 16 * p->nsm;
-    const UnsplitShape sh = g_tune[p->d.riemann & (TUNE_SLOTS - 1)];
+    const UnsplitShape sh = tuned_shape(p->d.riemann, true);
     if (sh.variant != 0 || sh.rows != 0) return false;  // the caller asked for a marching shape
     return tiles <= (half ? 7 : 12) * p->nsm;
 }
@@ -2294,6 +2306,20 @@ int run_selftest(void (*kernel)(int, unsigned long long, unsigned long long*), c
 }
 }  // namespace
 
+namespace {
+int tune_set(int riemann, int variant, int rows, int flag) {
+    int me = 0, mw = 0;
+    if (rp_shape(riemann, &me, &mw) != 0) return fail(CLAW2_EINVAL, "unknown Riemann solver id %d", riemann);
+    if (variant < 0 || (variant > 4 && variant != 8))
+        return fail(CLAW2_EINVAL, "variant must be 0..4 or 8 (got %d)", variant);
+    if (rows < 0 || rows > 4096) return fail(CLAW2_EINVAL, "rows must be 0..4096 (got %d)", rows);
+    g_tune[riemann & (TUNE_SLOTS - 1)].variant = variant | flag;
+    g_tune[riemann & (TUNE_SLOTS - 1)].rows = rows;
+    ++g_tune_gen;
+    return CLAW2_OK;
+}
+}  // namespace
+
 extern "C" {
 
 int claw2_selftest_sqrt(int device, int n, unsigned long long seed, double* max_ulp) {
@@ -2340,22 +2366,13 @@ int claw2_selftest_lpt(int device, int n, unsigned long long seed, int* mismatch
     return CLAW2_OK;
 }
 
-int claw2_tune_set(int riemann, int variant, int rows) {
-    int me = 0, mw = 0;
-    if (rp_shape(riemann, &me, &mw) != 0) return fail(CLAW2_EINVAL, "unknown Riemann solver id %d", riemann);
-    if (variant < 0 || (variant > 4 && variant != 8))
-        return fail(CLAW2_EINVAL, "variant must be 0..4 or 8 (got %d)", variant);
-    if (rows < 0 || rows > 4096) return fail(CLAW2_EINVAL, "rows must be 0..4096 (got %d)", rows);
-    g_tune[riemann & (TUNE_SLOTS - 1)].variant = variant;
-    g_tune[riemann & (TUNE_SLOTS - 1)].rows = rows;
-    ++g_tune_gen;
-    return CLAW2_OK;
-}
+int claw2_tune_set(int riemann, int variant, int rows) { return tune_set(riemann, variant, rows, 0); }
+int claw2_tune_set_step(int riemann, int variant, int rows) { return tune_set(riemann, variant, rows, TUNE_STEP_ONLY); }
 
 int claw2_tune_get(int riemann, int* variant, int* rows) {
     int me = 0, mw = 0;
     if (rp_shape(riemann, &me, &mw) != 0 || !variant || !rows) return fail(CLAW2_EINVAL, "bad arguments");
-    *variant = g_tune[riemann & (TUNE_SLOTS - 1)].variant;
+    *variant = g_tune[riemann & (TUNE_SLOTS - 1)].variant & ~TUNE_STEP_ONLY;
     *rows = g_tune[riemann & (TUNE_SLOTS - 1)].rows;
     return CLAW2_OK;
 }

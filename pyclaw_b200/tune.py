@@ -4,7 +4,8 @@ For one device patch (a problem size and Riemann solver) it times the step
 kernel -- CUDA events recorded by the library on the patch's stream -- for
 each compiled register budget and a set of row-block heights, rejecting every
 trial step so the state does not change, and installs the fastest shape with
-claw2_tune_set.  Results are cached per (solver id, mx, my) for the process.
+claw2_tune_set_step: the device time loop (other kernels, and a cooperative
+one on small grids) keeps its own choice.  Results are cached per (solver id, mx, my) for the process.
 """
 import ctypes
 import statistics
@@ -18,6 +19,11 @@ _cache = {}
 
 def set_shape(rp_id, variant, rows):
     _lib.check(_lib.load().claw2_tune_set(int(rp_id), int(variant), int(rows)))
+
+
+def set_step_shape(rp_id, variant, rows):
+    """As set_shape, but not for the device time loop."""
+    _lib.check(_lib.load().claw2_tune_set_step(int(rp_id), int(variant), int(rows)))
 
 
 def get_shape(rp_id):
@@ -35,13 +41,13 @@ def autotune(patch, dt, reps=5, rows=ROWS, variants=VARIANTS, before_step=None):
     d = patch.desc
     key = (d.riemann, d.mx, d.my)
     if key in _cache:
-        set_shape(d.riemann, *_cache[key][0])
+        set_step_shape(d.riemann, *_cache[key][0])
         return _cache[key]
     patch.set_timing(True)
     results = {}
     for v in variants:
         for r in rows:
-            set_shape(d.riemann, v, r)
+            set_step_shape(d.riemann, v, r)
             times = []
             for _ in range(reps + 1):
                 if before_step is not None:
@@ -51,6 +57,6 @@ def autotune(patch, dt, reps=5, rows=ROWS, variants=VARIANTS, before_step=None):
                 times.append(patch.kernel_ms())
             results[(v, r)] = statistics.median(times[1:])
     best = min(results, key=results.get)
-    set_shape(d.riemann, *best)
+    set_step_shape(d.riemann, *best)
     _cache[key] = (best, results)
     return best, results

@@ -82,6 +82,17 @@ __device__ __forceinline__ double rcp_nr(double a) {
     return (e == e) ? r : r0;
 }
 
+// n / a from r = rcp_nr(a): the product n r and one correction by its residual
+// n - q a, formed by one fused multiply-add, times r (Markstein, as above).  The product
+// alone carries the reciprocal's ulp and its own rounding; corrected, the quotient differs
+// from the IEEE one where that is a near tie.  A zero, infinite or NaN residual's
+// special cases return the product.
+__device__ __forceinline__ double quot_nr(double n, double a, double r) {
+    const double q = n * r;
+    const double c = fma(fma(-q, a, n), r, q);
+    return (c == c) ? c : q;
+}
+
 // sqrt(x) by Goldschmidt's coupled iteration from PTX's approximate
 // reciprocal square root y ~ 1/sqrt(x) (rsqrt.approx.ftz.f64): g = x y ~
 // sqrt(x) and h = y/2 are refined together, g <- g + g r, h <- h + h r with

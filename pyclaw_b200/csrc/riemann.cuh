@@ -1042,9 +1042,9 @@ struct RPVcAcoustics {
         const double zr = cR[ZZ], zl = cL[ZZ];
         const double delta1 = cR[0] - cL[0];
         const double delta2 = cR[MU] - cL[MU];
-        const double iz = rcp_nr(zl + zr);
-        f.alpha[0] = (-delta1 + zr * delta2) * iz;
-        f.alpha[1] = (delta1 + zl * delta2) * iz;
+        const double z = zl + zr, iz = rcp_nr(z);
+        f.alpha[0] = quot_nr(-delta1 + zr * delta2, z, iz);
+        f.alpha[1] = quot_nr(delta1 + zl * delta2, z, iz);
         f.zl = zl; f.zr = zr; f.cl = cL[CC]; f.cr = cR[CC];
         double w[MWAVES][MEQN], s[MWAVES];
         waves<IXY>(f, p, w);
@@ -1063,8 +1063,9 @@ struct RPVcAcoustics {
                                                     double (&bm)[MEQN], double (&bp)[MEQN]) {
         constexpr int MU = Dir<IXY>::MU, MV = Dir<IXY>::MV;
         const double zm = cm[ZZ], zz = c0[ZZ], zp = cp[ZZ];
-        const double a1 = (-asdq[0] + asdq[MV] * zz) * rcp_nr(zm + zz);
-        const double a2 = (asdq[0] + asdq[MV] * zz) * rcp_nr(zz + zp);
+        const double z1 = zm + zz, z2 = zz + zp;
+        const double a1 = quot_nr(-asdq[0] + asdq[MV] * zz, z1, rcp_nr(z1));
+        const double a2 = quot_nr(asdq[0] + asdq[MV] * zz, z2, rcp_nr(z2));
         bm[0] = cm[CC] * a1 * zm; bm[MU] = 0.0; bm[MV] = -cm[CC] * a1;
         bp[0] = cp[CC] * a2 * zp; bp[MU] = 0.0; bp[MV] = cp[CC] * a2;
     }

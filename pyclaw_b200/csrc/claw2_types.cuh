@@ -85,12 +85,11 @@ __device__ __forceinline__ double rcp_nr(double a) {
 // n / a from r = rcp_nr(a): the product n r and one correction by its residual
 // n - q a, formed by one fused multiply-add, times r (Markstein, as above).  The product
 // alone carries the reciprocal's ulp and its own rounding; corrected, the quotient differs
-// from the IEEE one where that is a near tie.  A zero, infinite or NaN residual's
-// special cases return the product.
+// from the IEEE one only where that is a near tie.  For normal a: where r is infinite
+// or zero (a zero, subnormal or infinite) the result is a NaN.
 __device__ __forceinline__ double quot_nr(double n, double a, double r) {
     const double q = n * r;
-    const double c = fma(fma(-q, a, n), r, q);
-    return (c == c) ? c : q;
+    return fma(fma(-q, a, n), r, q);
 }
 
 // sqrt(x) by Goldschmidt's coupled iteration from PTX's approximate

@@ -38,13 +38,20 @@ N = 1024
 MEQN = 4
 BYTES_PER_CELL = 2 * MEQN * 8  # read q^n + write q^{n+1}, FP64
 WORKLOAD = "euler_quadrants_roe_1024x1024_unsplit_trans_cor_mc"
-# One ncu capture of the step kernel on this workload (profiles/k_step_unsplit_euler_roe_1024.md):
-# dram__bytes_read.sum + dram__bytes_write.sum per launch, and the FP64 pipe's busy fraction.
-# The launch's 33.5 MB of output stays in L2 while it runs, so DRAM shows the reads only.
-# (Captured at three blocks per SM, H = 16, before the eigenvector coordinates: the bytes are the
-# same in every shape, the pipe's share moves with the shape.)
-NCU_TRAFFIC_BYTES = {1024: 34.801e6 + 0.926e6}
-NCU_FP64_PIPE_ACTIVE = {1024: 0.435}
+# ncu captures of the step kernel on this workload (profiles/kernel_counters.md), by grid size,
+# launch variant and row height: dram__bytes_read.sum + dram__bytes_write.sum per launch (the
+# launch's 33.5 MB of output stays in L2 while it runs, so DRAM shows the reads only), the FP64
+# pipe's busy fraction and the warps active per SM.
+NCU_CAPTURES = {
+    (1024, 0, 28): {"traffic": 34.265e6 + 0.366e6, "fp64_pipe_active": 0.374, "warps_per_sm": 6.9},
+    (1024, 1, 18): {"traffic": 34.503e6 + 0.765e6, "fp64_pipe_active": 0.399, "warps_per_sm": 10.0},
+}
+
+
+def captured(n, shape):
+    """The capture of the kernel a run of this grid size and launch shape times: {} for a shape
+    that was not captured."""
+    return NCU_CAPTURES.get((n,) + tuple(shape), {})
 
 
 def step_kernel_name(variant):
@@ -278,8 +285,9 @@ def time_patch(patch, dt, steps, flush, stream):
 def batched_workload(n_instances=512, steps=100, plain=True):
     """The batched form: n independent Euler quadrant problems of uneven size
     (side 64..512), 100 steps with per-problem dt; aggregate cell-updates/s of
-    the graph-captured persistent form and (plain=True) of the plain
-    per-problem loop."""
+    the graph-captured form over all tiles (graph_persistent, a name from when
+    its kernel was persistent; persistent_grid: the CTAs resident at once) and
+    (plain=True) of the plain per-problem loop."""
     import numpy as np
     from pyclaw_b200 import batch as pb, workloads
     claws, sides = workloads.batched_quadrants(n_instances)
@@ -296,7 +304,7 @@ def batched_workload(n_instances=512, steps=100, plain=True):
         if mode == 2:
             # the plain loop launches each problem alone: give every launch the
             # single-problem heuristic shape (most CTAs per launch), not the
-            # row heights tuned for the persistent kernel
+            # row heights tuned for the batch as a whole
             bat.set_rows(np.zeros(n_instances, dtype=np.intc))
         bat.upload()
         bat.set_time(dt0, 0.0, 1e99)
@@ -753,21 +761,21 @@ def run_ours(args):
                                                                  for k, v in sorted(trials.items())}},
                                   "state": "quadrant problem advanced to t=%g before warm-up" % args.pre_t}),
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                             "frac": achieved / peaks["hbm_gbs"], "traffic": NCU_TRAFFIC_BYTES.get(n),
-                             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch "
-                                               "(profiles/k_step_unsplit_euler_roe_1024.md)",
+                             "frac": achieved / peaks["hbm_gbs"], "traffic": captured(n, shape).get("traffic"),
+                             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch of "
+                                               "this shape (profiles/kernel_counters.md); null: shape not captured",
                              "peak_source": "%s (MEASURED_PEAKS.json hbm_gbs)" % peak_src,
                              "kernel": "%s (launch variant %d, H = %d)" % (step_kernel_name(shape[0]), shape[0],
                                                                            shape[1]),
                              "kernel_ms": kms,
                              "algorithmic_bytes_per_launch": cells * BYTES_PER_CELL,
                              "fp64_probe_tflops": fp64.value,
-                             "fp64_pipe_active_ncu": NCU_FP64_PIPE_ACTIVE.get(n),
-                             "note": "FP64-latency-bound kernel (10.8 warps/SM at the tuned 3-CTA shape, "
-                                     "dependency waits the top stall): ~870 FP64 instructions per developed "
-                                     "cell-update cap it near 2.1e10 cell-updates/s (21% of HBM) on this part; "
-                                     "warps whose interfaces all have equal cells on both sides (37% of this "
-                                     "state's) skip the finish"},
+                             "fp64_pipe_active_ncu": captured(n, shape).get("fp64_pipe_active"),
+                             "warps_per_sm_ncu": captured(n, shape).get("warps_per_sm"),
+                             "note": "FP64-latency-bound kernel (dependency waits the top stall): ~630 FP64 "
+                                     "instructions per developed cell-update cap it near 3.0e10 cell-updates/s "
+                                     "(29% of HBM) on this part; warps whose interfaces all have equal cells on "
+                                     "both sides (37% of this state's) skip the finish"},
                 "cpu_baseline": cpu, "e2e": e2e, "clocks": clk.summary(),
                 "secondary": secondary,
                 "gpu_launches": int(launches1.value - launches0.value)}

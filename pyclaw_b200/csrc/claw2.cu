@@ -203,8 +203,8 @@ void smem_attr(K kernel, int bytes, unsigned long long& done) {
 
 // Launch shapes of the unsplit kernel.  A variant fixes the register budget
 // (blocks per SM the kernel is compiled for); `rows` is the row-block height
-// (0 = heuristic).  Chosen per call by the tuning table (claw2_tune_set /
-// claw2_autotune) or the heuristic default.
+// (0 = heuristic).  Chosen per call by the tuning table (claw2_tune_set,
+// pyclaw_b200.tune) or the heuristic default.
 struct UnsplitShape {
     int variant;  // bit 0: 3 blocks/SM (register cap) instead of 2; bit 1: TMA row staging
                   // (4 and 8 once named two other tiles: accepted, run as 0)
@@ -1111,7 +1111,7 @@ namespace {
 
 // Buffers of the longest-first schedule for n tiles of height H; a new
 // tiling starts from the identity order.  Returns non-OK (no schedule) when
-// the tiling is too large for the one-CTA sort or the buffers cannot be had.
+// there are more tiles than k_lpt_order's shared memory holds, or the buffers cannot be had.
 int lpt_prepare(claw2_patch* p, int n, int H) {
     if (n < 1 || n > LPT_MAX_TILES) return CLAW2_EINVAL;
     if (n > p->tile_cap) {
@@ -1630,7 +1630,9 @@ int patch_enqueue_step(claw2_patch* p, double dt, int part = 0) {
         dispatch<SplitF>(p->d.riemann, ax, ay, p->st, 3);
         p->step_launches += 2;
     } else {
-        // a schedule only matters when the tiles outnumber the CTA slots (2 per SM)
+        // (no schedule for tiles that are all alone on an SM, or in pairs.  Where they are one wave of
+        // three per SM the order still decides which ones share an SM: 24 steps of the 1024^2
+        // quadrant loop 2.66 ms, 2.69 without; flows active everywhere 1% the other way)
         if (ns * nb > 2 * p->nsm && lpt_prepare(p, ns * nb, H) == CLAW2_OK) {
             lpt_n = ns * nb;
             a.H = H;

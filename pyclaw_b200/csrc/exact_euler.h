@@ -229,12 +229,8 @@ struct Fan {
 // density in units of 1e-17 rho, for ratios within 15% of one, within 60%, over four decades:
 // 6.7, 6.9, 9.8; by a power, at the p* of differences of rounded powers, 10.8, 10.6,
 // 9.9; by the product of rounded factors there 19.7, 18.8, 15.9.  (What this costs, with
-// prefun's difference: six steps at 1024^2 2.14 -> 2.32 ms.)
-// A side that ends on the rarefaction branch after its last evaluation on the shock
-// branch (e near 2) is within the tolerance of p_K, where e = g1 (p*/p_K - 1) to
-// second order.
+// prefun's difference: six steps at 1024^2 2.14 -> 2.23 ms.)
 EX_HD void rarefied(const Gas& G, double ps, double rk, double pk, double ck, double e, double& rs, double& cm) {
-    if (e > 1.0) e = G.g1 * ((ps - pk) * ex_rcp(pk));
     const double x = 1.0 + e;
     const bool weak = e > -0.05;
     const double t = pk * x, den = t * x, r = ex_rcp(den);
@@ -247,11 +243,12 @@ EX_HD void rarefied(const Gas& G, double ps, double rk, double pk, double ck, do
 
 EX_HD Fan fan(const Gas& G, double rl, double ul, double pl, double cl, double rr, double ur, double pr, double cr,
               double ps, double us, double xl, double xr) {
+    // (A wave is what star's last evaluation took it for.  Where its last step went past p_K,
+    // within the tolerance, the shock's relations and the isentrope differ by the cube of
+    // that step.)
     Fan F;
-    // (exactly 1 for ps equal to the side's pressure, as a quotient would be:
-    // the record of two equal states stays the zero-jump shortcut's)
-    const double pml = (ps == pl) ? 1.0 : ps * ex_rcp(pl), pmr = (ps == pr) ? 1.0 : ps * ex_rcp(pr);
-    if (ps > pl) {
+    if (xl > 1.0) {
+        const double pml = ps * ex_rcp(pl);
         F.rsl = rl * (pml + G.g6) * ex_rcp(pml * G.g6 + 1.0);
         F.s1 = ul - cl * ex_sqrt(G.g2 * pml + G.g1);
         F.cml = 0.0;
@@ -259,7 +256,8 @@ EX_HD Fan fan(const Gas& G, double rl, double ul, double pl, double cl, double r
         rarefied(G, ps, rl, pl, cl, xl, F.rsl, F.cml);
         F.s1 = 0.5 * ((ul - cl) + (us - F.cml));
     }
-    if (ps > pr) {
+    if (xr > 1.0) {
+        const double pmr = ps * ex_rcp(pr);
         F.rsr = rr * (pmr + G.g6) * ex_rcp(pmr * G.g6 + 1.0);
         F.s3 = ur + cr * ex_sqrt(G.g2 * pmr + G.g1);
         F.cmr = 0.0;
@@ -277,7 +275,7 @@ EX_HD void sample0(const Gas& G, double rl, double ul, double pl, double cl, dou
     const double s = 0.0;
     left = s <= us;
     if (left) {
-        if (ps <= pl) {
+        if (F.cml > 0.0) {  // (a rarefaction)
             const double shl = ul - cl;
             if (s <= shl) { r = rl; u = ul; p = pl; return; }
             const double stl = us - F.cml;
@@ -294,7 +292,7 @@ EX_HD void sample0(const Gas& G, double rl, double ul, double pl, double cl, dou
             else { r = F.rsl; u = us; p = ps; }
         }
     } else {
-        if (ps > pr) {
+        if (!(F.cmr > 0.0)) {
             const double sr = F.s3;
             if (s >= sr) { r = rr; u = ur; p = pr; }
             else { r = F.rsr; u = us; p = ps; }

@@ -38,7 +38,7 @@ N = 1024
 MEQN = 4
 BYTES_PER_CELL = 2 * MEQN * 8  # read q^n + write q^{n+1}, FP64
 WORKLOAD = "euler_quadrants_roe_1024x1024_unsplit_trans_cor_mc"
-# ncu captures of the step kernel on this workload (profiles/kernel_counters.md), by grid size,
+# ncu captures of the step kernel on this workload, by grid size,
 # launch variant and row height: dram__bytes_read.sum + dram__bytes_write.sum per launch (the
 # launch's 33.5 MB of output stays in L2 while it runs, so DRAM shows the reads only), the FP64
 # pipe's busy fraction and the warps active per SM.

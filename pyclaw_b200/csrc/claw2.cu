@@ -966,7 +966,10 @@ int claw2_mlp_train(claw2_mlp* m, int epochs, int batch, float lr, float* last_l
         CUDA_TRY(cudaMemsetAsync(m->loss, 0, 4, m->st));
         int fault = 0;
         for (long long b = 0; b < nb;) {
-            const int n = (int)std::min<long long>(nb - b, 4096);  // (tens of milliseconds per launch)
+            // (about 20 ms per launch, which holds every SM: 9.5 us per minibatch and 0.4 ns per
+            // sample; by 4096 minibatches whatever their size, 0.15 s at 65536)
+            const int most = std::max(1, (int)(0.02 / (9.5e-6 + 0.4e-9 * batch)));
+            const int n = (int)std::min<long long>(nb - b, most);
             if (mlp_epoch_launch(m, b, n, batch, e * nb + b, epochs * nb, lr) == cudaSuccess) {
                 CUDA_TRY(cudaMemcpyAsync(&fault, &m->ctl->fault, 4, cudaMemcpyDeviceToHost, m->st));
                 CUDA_TRY(cudaStreamSynchronize(m->st));

@@ -345,7 +345,7 @@ struct ShapeF {
 template <class RP, int MB, bool EVO>
 void launch_unsplit_v(const StepArgs& a, cudaStream_t st, const CUtensorMap* tm, const CUtensorMap* tm1) {
     StepArgs b = a;
-    if (b.tile_order == nullptr) {  // a caller with a schedule has fixed H and nstrips already
+    if (b.H <= 0) {  // (a patch has worked out its tiling already)
         int ns, H, nb;
         unsplit_tiling(RP::ID, a.capa != nullptr, EVO, a.L.mx, a.L.my, ns, H, nb);
         b.H = H;
@@ -460,7 +460,10 @@ struct KeepsRestF {
 // each SM) march H + 3 rows in as many waves as the tiles need, so a tile count
 // just over a multiple of the slots is a wave nearly empty (24 steps at 1024^2
 // Euler with two CTAs per SM: H = 21, 1.5 waves, 3.08 ms; 1 wave of three per SM
-// 2.75 ms).  The exact solver's tiles differ too much in their Newton work for
+// 2.75 ms).  Up to three CTAs on an SM march as fast as one; four or five (the smallest
+// records) share it, 1.27 and 1.58 times a row: counted as free, shorter blocks for their
+// slots cost 5% (variable advection at 700 x 600 16.4 -> 17.3 us), counted not at all, order-1
+// advection at 2000 x 1715 takes 47 us for 37.  The exact solver's tiles differ too much in their Newton work for
 // that count (one wave waits for its slowest tile: six steps at 1024^2 4.69 ms
 // against 3.45; three at 2048^2 4.58 ms with H = 64, 4.01 with 28): taken longest
 // first, their march is list_march's, and at most that of three blocks per SM.  Best
@@ -472,7 +475,7 @@ void unsplit_tiling(int riemann, bool capa, bool evo, int mx, int my, int& nstri
     int rows = 0, per_sm = 2;
     dispatch<ShapeF>(riemann, capa, evo, &rows, &per_sm);
     nstrips = (mx + W - 1) / W;
-    const int slots = device_sms() * per_sm;
+    const int nsm = device_sms(), slots = nsm * per_sm;
     if (rows > 0) {
         H = rows;
     } else if (riemann == CLAW2_RP_EULER_EXACT) {
@@ -481,14 +484,16 @@ void unsplit_tiling(int riemann, bool capa, bool evo, int mx, int my, int& nstri
             if (list_march((long long)nstrips * (my + 3 * ((my + h - 1) / h)), slots, h) <
                 list_march((long long)nstrips * (my + 3 * ((my + H - 1) / H)), slots, H))
                 H = h;
-        H = std::min(H, pick_rows(nstrips, my, device_sms()));
+        H = std::min(H, pick_rows(nstrips, my, nsm));
     } else {
-        long long best = 0;
+        double best = 0.0;
         H = 2;
         for (int h = 2; h <= 64; ++h) {
             const long long tiles = (long long)nstrips * ((my + h - 1) / h);
-            const long long march = (tiles + slots - 1) / slots * (std::min(h, my) + 3);
-            if (best == 0 || march < best) {
+            const int together = (int)std::min<long long>(per_sm, (tiles + nsm - 1) / nsm);
+            const double row = together > 3 ? 0.95 / 3.0 * together : 1.0;
+            const double march = row * (double)((tiles + slots - 1) / slots * (std::min(h, my) + 3));
+            if (best == 0.0 || march < best) {
                 best = march;
                 H = h;
             }
@@ -1590,9 +1595,9 @@ int patch_enqueue_step(claw2_patch* p, double dt, int part = 0) {
         ++p->step_launches;
     }
     StepArgs a = patch_args(p, dt);
+    a.H = H;
+    a.nstrips = ns;
     if (part != 0) {
-        a.H = H;
-        a.nstrips = ns;
         if (part == 1) {  // row blocks 1 .. b_hi
             a.tile_offset = ns;
             a.tile_count = ns * b_hi;
@@ -1638,8 +1643,6 @@ int patch_enqueue_step(claw2_patch* p, double dt, int part = 0) {
         // quadrant loop 2.66 ms, 2.69 without; flows active everywhere 1% the other way)
         if (ns * nb > 2 * p->nsm && lpt_prepare(p, ns * nb, H) == CLAW2_OK) {
             lpt_n = ns * nb;
-            a.H = H;
-            a.nstrips = ns;
             a.tile_order = p->tile_order;
             a.tile_cost = p->tile_cost;
         }
@@ -1834,10 +1837,10 @@ int evolve_enqueue_attempt(claw2_patch* p, int c, int rest) {
     } else {
         int ns, H, nb;
         unsplit_tiling(p->d.riemann, p->d.mcapa > 0, true, p->L.mx, p->L.my, ns, H, nb);
+        a.H = H;
+        a.nstrips = ns;
         if (ns * nb > 2 * p->nsm && lpt_prepare(p, ns * nb, H) == CLAW2_OK) {
             lpt_n = ns * nb;
-            a.H = H;
-            a.nstrips = ns;
             a.tile_order = p->tile_order;
             a.tile_cost = p->tile_cost;
         }
